@@ -121,6 +121,19 @@ cudaStream_t capture_side_stream() {
   return streams[dev];
 }
 
+std::mutex& coop_mutex() {
+  static std::mutex mu;
+  return mu;
+}
+
+cudaEvent_t coop_event(int dev) {
+  static cudaEvent_t ev[64] = {};
+  if (dev < 0 || dev >= 64) return nullptr;
+  if (!ev[dev] && cudaEventCreateWithFlags(&ev[dev], cudaEventDisableTiming) != cudaSuccess)
+    ev[dev] = nullptr;
+  return ev[dev];
+}
+
 }  // namespace gdn
 
 extern "C" const char* gdn_version(void) { return "gradenna_b200 0.1 (sm_100a)"; }

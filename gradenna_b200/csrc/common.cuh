@@ -6,6 +6,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -79,6 +80,11 @@ class LoopTimer {
 cudaStream_t capture_stream();
 // A second private stream per device for parallel branches inside captures.
 cudaStream_t capture_side_stream();
+
+// Cooperative launches of this process on one device follow one another: the
+// lock is held while a launch waits for the event and records it anew.
+std::mutex& coop_mutex();
+cudaEvent_t coop_event(int dev);
 
 template <typename T>
 struct Cplx;

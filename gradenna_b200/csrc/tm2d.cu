@@ -76,9 +76,12 @@ struct Pt {
 };
 
 // A DFT monitor resolved against the grid: box [lo0, lo0+h) x [lo1, lo1+w)
-// of component comp, stored at `off` in every monitor-ring slot.
+// of component comp, stored at `off` in every monitor-ring slot, `pitch`
+// values a row of which the first `pad` and the last are unused (0 and w for
+// the tile and march kernels; for the resident ones column j of the grid is at
+// a ring index that is j modulo 4).
 struct MonD {
-  int comp, lo0, lo1, h, w, pad;
+  int comp, lo0, lo1, h, w, pad, pitch, unused;
   long long count, off;
   void* out;
 };
@@ -620,6 +623,9 @@ __global__ void __launch_bounds__(NT) tm_tb_batch(const Dev<T>* devs, const int2
   tb_body<T, TB, TI, TJ, NT, GEN>(*reinterpret_cast<const Dev<T>*>(sdev), w.y, sub0, nsub);
 }
 
+// The register-resident kernels (defined in this namespace).
+#include "tm2d_res.cuh"
+
 // ---------------------------------------------------------------------------
 // Running DFT fold over `cnt` monitor-ring slots (fdtd2d.py:453-458): for
 // each monitored cell, acc_k += sum_t ph[n0+t, k] x_t, partial sums in A.
@@ -768,23 +774,26 @@ __global__ void tm_pad_in(const T* src, T* dst, int nx, int ny, int ld) {
   }
 }
 
-// Copy the final state slot into the caller's unpadded ez/hx/hy.
+// Copy the final state slot into the caller's unpadded ez/hx/hy. `err` (or
+// null): set when a resident tile gave up on a wait; the results are then NaN.
 template <typename T>
 __global__ void tm_copy_out(const T* slot, long long plane, int nx, int ny, int ld, T* ez, T* hx,
-                            T* hy) {
+                            T* hy, const int* err) {
+  const T bad = err && *err ? T(NAN) : T(0);
   const long long total = (long long)nx * ny;
   for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int i = int(g / ny), j = int(g - (long long)i * ny);
     const long long c = cell_at(ld, i, j);
-    ez[g] = slot[c];
-    if (j < ny - 1) hx[(long long)i * (ny - 1) + j] = slot[plane + c];
-    if (i < nx - 1) hy[g] = slot[2 * plane + c];
+    ez[g] = bad == bad ? slot[c] : bad;
+    if (j < ny - 1) hx[(long long)i * (ny - 1) + j] = bad == bad ? slot[plane + c] : bad;
+    if (i < nx - 1) hy[g] = bad == bad ? slot[2 * plane + c] : bad;
   }
 }
 
 template <typename C>
-__global__ void tm_dft_scale(C* a, long long count, double s) {
+__global__ void tm_dft_scale(C* a, long long count, double s, const int* err) {
+  if (err && *err) s = NAN;
   for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < count;
        g += (long long)gridDim.x * blockDim.x) {
     C v = a[g];
@@ -798,16 +807,141 @@ __global__ void tm_dft_scale(C* a, long long count, double s) {
 // Host side
 // ---------------------------------------------------------------------------
 
+// ---- plan of the resident kernels: rectangles ----
+
+struct ShapeInfo {
+  int ti, tj, eh, ew, nt, gen_elems;  // gen_elems: shared elements before psi
+};
+template <class S>
+static ShapeInfo shape_info() {
+  return ShapeInfo{S::TI, S::TJ, S::EH, S::EW, S::NT, S::O_GEN + S::KE};
+}
+// Shape of a kind's interior (general) rectangles.
+static ShapeInfo kind_shape(size_t esize, int kind, bool gen) {
+  if (esize == sizeof(double)) {
+    switch (kind) {
+      case 0: return shape_info<res::F64A>();
+      case 1: return gen ? shape_info<res::F64A>() : shape_info<res::F64B>();
+      default: return gen ? shape_info<res::F64CG>() : shape_info<res::F64C>();
+    }
+  }
+  switch (kind) {
+    case 0: return shape_info<res::F32A>();
+    case 1: return gen ? shape_info<res::F32A>() : shape_info<res::F32B>();
+    case 2: return gen ? shape_info<res::F32CG>() : shape_info<res::F32C>();
+    case 3: return gen ? shape_info<res::F32DG>() : shape_info<res::F32D>();
+    default: return gen ? shape_info<res::F32EG>() : shape_info<res::F32E>();
+  }
+}
+static int kinds(size_t esize) { return esize == sizeof(float) ? res::NKIND : 3; }
+
+// A class region cut into nr x nc pieces of at most ph x pw cells; its first
+// rectangle's index.
+struct Region {
+  int i0, j0, h, w, gen, ph, pw, nr, nc, first;
+};
+struct Plan {
+  std::vector<Region> regions;
+  int n_rects = 0;
+  size_t smem = 0;  // dynamic shared memory of a CTA
+  bool fits = false;
+};
+
+static int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
+    cudaGetLastError();
+    return 148;
+  }
+  return sms;
+}
+
+// Rectangles of a grid under `kind`. The interior tiles of configuration c
+// form a rectangle of cells; the rest is general: a strip of rows above and
+// below it, columns left and right.
+static Plan make_plan(const GdnTmParams* p, size_t esize, const Cfg& c, int kind) {
+  const int m = p->npml, nx = p->nx, ny = p->ny;
+  auto span = [&](int len, int t, int halo, int* lo, int* hi) {
+    *lo = *hi = 0;
+    for (int q = 0; q * t < len; ++q)
+      if (q * t - halo >= m + 1 && (q + 1) * t + halo - 1 <= len - 2 - m) {
+        if (*hi == 0) *lo = q * t;
+        *hi = (q + 1) * t;
+      }
+  };
+  int r0, r1, c0, c1;
+  span(nx, c.ti, c.tb, &r0, &r1);
+  span(ny, c.tj, HJ, &c0, &c1);
+  Plan pl;
+  auto add = [&](int i0, int j0, int h, int w, int gen) {
+    if (h <= 0 || w <= 0) return;
+    const ShapeInfo s = kind_shape(esize, kind, gen != 0);
+    Region g{i0, j0, h, w, gen, 0, 0, int(div_up(h, s.ti)), int(div_up(w, s.tj)), pl.n_rects};
+    g.ph = int(div_up(h, g.nr));
+    g.pw = int(std::min<long long>(s.tj, div_up(div_up(w, g.nc), 4) * 4));  // vectors stay aligned
+    g.nr = int(div_up(h, g.ph));
+    g.nc = int(div_up(w, g.pw));
+    pl.n_rects += g.nr * g.nc;
+    for (int r = 0; r < g.nr; ++r)
+      for (int q = 0; q < g.nc; ++q) {
+        size_t el = size_t(s.gen_elems);
+        if (gen) {
+          const res::Slab sx = res::slab_range(i0 + r * g.ph - res::TB, s.eh, nx, m);
+          const res::Slab sy = res::slab_range(j0 + q * g.pw - res::TB, s.ew, ny, m);
+          el += size_t(res::psi_elems(sx, sy, s.eh, s.ew));
+        }
+        pl.smem = std::max(pl.smem, el * esize);
+      }
+    pl.regions.push_back(g);
+  };
+  if (r1 == 0 || c1 == 0) {
+    add(0, 0, nx, ny, 1);
+  } else {
+    add(0, 0, r0, ny, 1);
+    add(r1, 0, nx - r1, ny, 1);
+    add(r0, 0, r1 - r0, c0, 1);
+    add(r0, c1, r1 - r0, ny - c1, 1);
+    add(r0, c0, r1 - r0, c1 - c0, 0);
+  }
+  pl.fits = pl.smem <= size_t(220) << 10;
+  return pl;
+}
+
+// Kind of a single run: the smallest whose rectangles all have an SM of their
+// own; -1: none (the tile kernels then). The line lies there because rectangles
+// wait for one another: with more of them than SMs the state would have to go
+// through memory every block. Tried with one launch a block, 1024 x 1024 f64
+// took 36 ms for 1000 steps where the tile kernels take 30. Batches keep the
+// tile kernels too: they fill the chip already (24 problems of 128^2 to 512^2,
+// gradients: 0.45 s; 0.49 s with resident launches one after another).
+static int choose_kind(const GdnTmParams* p, size_t esize, const Cfg& c, Plan* out) {
+  const int sms = sm_count();
+  for (int k = 0; k < kinds(esize); ++k) {
+    Plan pl = make_plan(p, esize, c, k);
+    if (pl.fits && pl.n_rects <= sms) {
+      *out = std::move(pl);
+      return k;
+    }
+  }
+  return -1;
+}
+
 struct Layout {
   Cfg cfg;
   // Row march (tm_march) instead of shared-memory tiles (tm_tb): then a
   // "tile" is one warp's strip segment, cfg.ti its owned rows and cfg.tj its
   // owned columns.
   bool march = false;
+  // Register-resident tiles (tm_res); seg = steps per segment.
+  bool res = false;
+  int seg = 0, kind = 0;
+  Plan plan;
   int ld = 0, rows = 0, tiles_x = 0, tiles_y = 0, n_tiles = 0, R = 32, n_gen = 0, n_int = 0;
   long long plane = 0, mon_cells = 0, n_mw = 0, n_mpts = 0;
   size_t state[2], ca, cb, psi[2], zero_end, tile_list, off[5], pts[5], mons, mw_off, mw, mring,
-      step, eacc, tasks, mpts, total;
+      step, eacc, tasks, mpts, xch, err, blob, pv, total;
+  size_t blob_bytes = 0;
 };
 
 // The row march is selected with GDN_TM_KERNEL=march (runs that record the
@@ -896,11 +1030,97 @@ static bool tile_is_interior(const GdnTmParams* p, const Cfg& c, int ty, int tx)
   return r0 >= m + 1 && r1 - 1 <= p->nx - 2 - m && c0 >= m + 1 && c1 - 1 <= p->ny - 2 - m;
 }
 
-// `ring_steps` > 0 forces the monitor-ring length (a multiple of TB).
+// Index of configuration c in its type's table (NCFG: the one-step shape).
+static int cfg_index_of(size_t esize, const Cfg& c) {
+  if (c.tb == 1) return NCFG;
+  const Cfg* t = esize == sizeof(float) ? kCfgF32 : kCfgF64;
+  for (int i = 0; i < NCFG; ++i)
+    if (t[i].tb == c.tb && t[i].ti == c.ti && t[i].tj == c.tj) return i;
+  return 0;
+}
+
+// Ring pitch of a monitor row for the resident kernels.
+static int ring_pitch(int lo1, int w) { return (lo1 % 4 + w + 3) / 4 * 4; }
+
+static long long padded_cells(const GdnTmParams* p, const GdnTmPoints* pts) {
+  long long c = 0;
+  for (const auto& b : monitor_boxes(p, pts)) c += (long long)b[3] * ring_pitch(b[2], b[4]);
+  return c;
+}
+
+// The resident kernels stand in for the two configurations that pick_cfg
+// chooses. They are used unless an environment variable asks for the tile or
+// march kernels (GDN_TM_KERNEL, GDN_TM_TILE), the energy is recorded every
+// step, or the monitors are so many that the DFT's partial sums would be
+// shorter than FOLD steps.
+static bool use_res(const GdnTmParams* p, const GdnTmPoints* pts, size_t esize, const Cfg& c) {
+  if (p->record_energy) return false;
+  const char* kind = getenv("GDN_TM_KERNEL");
+  const char* tile = getenv("GDN_TM_TILE");
+  if ((kind && kind[0] && kind[0] != 'r') || (tile && tile[0])) return false;
+  const int which = cfg_index_of(esize, c);
+  if (which != 1 && which != 2) return false;
+  if (p->n_freq > 0 && !pts && p->n_monitors > 0) return false;
+  // Counts of a thread's points are kept in 16 bits.
+  if (std::max({p->n_sources, p->n_mx, p->n_my, p->n_ports, p->n_probes}) > 65535) return false;
+  return padded_cells(p, pts) * res::FOLD * (long long)esize <= (2LL << 30);
+}
+
+// Calls f(region, r, q, index) for the rectangles that meet the cells [a0, a1)
+// x [b0, b1).
+template <typename F>
+static void rects_of(const Plan& pl, int a0, int a1, int b0, int b1, F&& f) {
+  for (const Region& g : pl.regions) {
+    const int ra = std::max(a0, g.i0), rb = std::min(a1, g.i0 + g.h);
+    const int ca = std::max(b0, g.j0), cb = std::min(b1, g.j0 + g.w);
+    if (ra >= rb || ca >= cb) continue;
+    for (int r = (ra - g.i0) / g.ph; r <= (rb - 1 - g.i0) / g.ph; ++r)
+      for (int q = (ca - g.j0) / g.pw; q <= (cb - 1 - g.j0) / g.pw; ++q) f(g, r, q, g.first + r * g.nc + q);
+  }
+}
+static res::Rect rect_at(const Region& g, int r, int q) {
+  const int i0 = g.i0 + r * g.ph, j0 = g.j0 + q * g.pw;
+  return res::Rect{i0, j0, std::min(g.ph, g.i0 + g.h - i0), std::min(g.pw, g.j0 + g.w - j0), g.gen};
+}
+
+// Bound on the copies of points in rectangles and their halos.
+static size_t res_copies(const Plan& pl, const GdnTmParams* p) {
+  const size_t np = size_t(p->n_sources) + p->n_mx + p->n_my + p->n_ports;
+  int small = 1 << 30;
+  for (const Region& g : pl.regions) small = std::min({small, g.ph, g.pw});
+  // Within TB cells of a point lie at most this many pieces a direction.
+  const size_t k = size_t(2 * res::TB / std::max(small, 1) + 2);
+  return np * std::min<size_t>(k * k, size_t(pl.n_rects)) + size_t(p->n_probes);
+}
+
+static long long injections(const GdnTmParams* p) {
+  return (long long)p->n_sources + p->n_mx + p->n_my + p->n_ports;
+}
+
+// Steps per segment: the ring within 256 MiB, the value table within 64 MiB.
+// Between segments the state goes through memory once (about 15 us at 1024^2
+// against 6 us a block), so a few hundred steps make that small.
+static int seg_steps(int n_steps, long long mon, long long inj, size_t esize) {
+  long long s = std::min<long long>(res::SEG_MAX, div_up(std::max(n_steps, 1), res::FOLD) * res::FOLD);
+  if (mon > 0) s = std::min<long long>(s, (256LL << 20) / (mon * (long long)esize));
+  if (inj > 0) s = std::min<long long>(s, (64LL << 20) / (inj * (long long)esize));
+  return int(std::max<long long>(res::FOLD, s / res::FOLD * res::FOLD));
+}
+
+// `ring_steps` > 0 forces the monitor-ring length (a multiple of TB; for the
+// resident kernels the segment length, a multiple of FOLD).
 static Layout make_layout(const GdnTmParams* p, const GdnTmPoints* pts, size_t esize,
-                          int ring_steps = 0, int force_cfg = -1) {
+                          int ring_steps = 0, int force_cfg = -1, bool allow_res = true) {
   Layout L;
   L.march = use_march(p, force_cfg);
+  if (!L.march && allow_res) {
+    const Cfg c = pick_cfg(p, esize, force_cfg);
+    L.res = use_res(p, pts, esize, c);
+    if (L.res) {
+      L.kind = choose_kind(p, esize, c, &L.plan);
+      L.res = L.kind >= 0;
+    }
+  }
   L.cfg = L.march ? (esize == sizeof(float) ? march_cfg<float>() : march_cfg<double>())
                   : pick_cfg(p, esize, force_cfg);
   const Cfg& c = L.cfg;
@@ -915,7 +1135,15 @@ static Layout make_layout(const GdnTmParams* p, const GdnTmPoints* pts, size_t e
   const bool mons_known = pts || p->n_monitors == 0;
   L.mon_cells = mons_known ? monitor_cells(p, pts) : 0;
   L.n_mw = mons_known ? monitor_parts(p, pts, c) : 0;
-  if (ring_steps > 0) {
+  if (L.res) {
+    L.n_mw = 0;
+    for (const auto& bx : monitor_boxes(p, pts))
+      rects_of(L.plan, bx[1], bx[1] + bx[3], bx[2], bx[2] + bx[4],
+               [&](const Region&, int, int, int) { ++L.n_mw; });
+    L.mon_cells = padded_cells(p, pts);
+    L.seg = ring_steps > 0 ? ring_steps : seg_steps(p->n_steps, L.mon_cells, injections(p), esize);
+    L.R = L.seg;
+  } else if (ring_steps > 0) {
     L.R = ring_steps;
   } else {
     const size_t budget = size_t(2) << 30;  // monitor ring budget: 2 GiB
@@ -938,9 +1166,30 @@ static Layout make_layout(const GdnTmParams* p, const GdnTmPoints* pts, size_t e
   L.cb = cv.take<char>(size_t(L.plane) * esize);
   for (int s = 0; s < 2; ++s) L.psi[s] = cv.take<char>(4 * size_t(L.plane) * esize);
   L.step = cv.take<int>(1);
+  if (L.res) {
+    L.xch = cv.take<uint4>(2 * size_t(L.plane) * (esize == sizeof(float) ? 3 : 7));
+    L.err = cv.take<int>(1);
+  }
   L.zero_end = cv.take<char>(0);
   L.tile_list = cv.take<int>(L.n_tiles);  // general tiles first, then interior
   const int counts[5] = {p->n_sources, p->n_ports, p->n_mx, p->n_my, p->n_probes};
+  if (L.res) {
+    // One blob, uploaded in one copy: descriptors, monitors, per-tile lists.
+    const size_t nr = size_t(L.plan.n_rects);
+    const size_t hdrs = std::min<size_t>(nr, res_copies(L.plan, p));
+    L.blob_bytes = sizeof(res::RDev<double>) + nr * sizeof(res::RTile) +
+                   size_t(std::max(p->n_monitors, 3)) * sizeof(MonD) + 2 * (nr + 1) * sizeof(int) +
+                   size_t(L.n_mw) * sizeof(MonW) +
+                   hdrs * size_t(kind_shape(esize, L.kind, false).nt) * sizeof(res::RHdr) +
+                   (hdrs + 1) * sizeof(int) +
+                   res_copies(L.plan, p) * (sizeof(res::RPt) + sizeof(int)) + 16 * 16;
+    L.blob = cv.take<char>(L.blob_bytes);
+    L.pv = cv.take<char>(std::max<size_t>(size_t(L.seg) * size_t(injections(p)), 1) * esize);
+    L.mring = cv.take<char>(std::max<size_t>(size_t(L.mon_cells) * L.seg, 1) * esize);
+    L.eacc = cv.take<double>(1);
+    L.total = cv.bytes();
+    return L;
+  }
   if (L.march) {
     // A point lies in the extended range of at most two segments x two strips.
     long long np = 0;
@@ -1099,6 +1348,14 @@ struct Run {
   std::vector<MTask> mtasks;
   std::vector<int> mtask_tiles;
   const MTask* tasks = nullptr;
+  // Resident kernels: descriptor, tiles (general first) and their device
+  // copies, dynamic shared memory of a CTA, give-up flag.
+  res::RDev<T> rd{};
+  std::vector<res::RTile> rtiles;
+  const res::RDev<T>* d_rd = nullptr;
+  const res::RTile* d_rtiles = nullptr;
+  size_t rsmem = 0;
+  int* err = nullptr;
 };
 
 template <typename T>
@@ -1110,6 +1367,12 @@ static int prepare_march(const GdnTmParams* p, const GdnTmPoints* pts, char* ws,
 template <typename T>
 static int prepare_common(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers* b,
                           char* ws, Run<T>& R, cudaStream_t stream);
+template <typename T>
+static int prepare_state(const GdnTmParams* p, const GdnTmBuffers* b, char* ws, Run<T>& R,
+                         cudaStream_t stream);
+template <typename T>
+static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers* b,
+                       char* ws, Run<T>& R, cudaStream_t stream);
 
 template <typename T, int TB, int TI, int TJ, bool GEN>
 static size_t tb_smem() {
@@ -1165,14 +1428,10 @@ static int set_kernel_attributes() {
   return GDN_OK;
 }
 
-// Index of a run's configuration in its type's table (NCFG: the one-step shape).
+// Index of a run's configuration in its type's table.
 template <typename T>
 static int cfg_index(const Cfg& c) {
-  if (c.tb == 1) return NCFG;
-  for (int i = 0; i < NCFG; ++i)
-    if (Kern<T>::c[i].tb == c.tb && Kern<T>::c[i].ti == c.ti && Kern<T>::c[i].tj == c.tj)
-      return i;
-  return 0;
+  return cfg_index_of(sizeof(T), c);
 }
 
 template <typename T, int TB, int TI, int TJ, int NT, bool GEN>
@@ -1352,6 +1611,10 @@ static int prepare(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuff
   d.step_base = R.step_base;
   R.eacc = reinterpret_cast<double*>(ws + L.eacc);
 
+  if (L.res) {
+    const int rs = prepare_res(p, pts, b, ws, R, stream);
+    return rs ? rs : prepare_state(p, b, ws, R, stream);
+  }
   d.mpts = reinterpret_cast<const MPt*>(ws + L.mpts);
   int st = L.march ? prepare_march(p, pts, ws, R, stream) : prepare_tiles(p, pts, ws, R, stream);
   if (st) return st;
@@ -1486,7 +1749,6 @@ static int prepare_common(const GdnTmParams* p, const GdnTmPoints* pts, const Gd
                           char* ws, Run<T>& R, cudaStream_t stream) {
   const Layout& L = R.L;
   Dev<T>& d = R.d;
-  const int nx = p->nx, ny = p->ny, N = p->n_steps;
 
   // Monitors (full grid when none are listed).
   const bool f64acc = p->dft_f64 != 0;
@@ -1499,7 +1761,7 @@ static int prepare_common(const GdnTmParams* p, const GdnTmPoints* pts, const Gd
     for (const auto& bx : monitor_boxes(p, pts)) {
       void* out = p->n_monitors == 0 ? full_out[k] : pts->monitors[k].out;
       const long long cnt = (long long)bx[3] * bx[4];
-      R.mons.push_back(MonD{bx[0], bx[1], bx[2], bx[3], bx[4], 0, cnt, off, out});
+      R.mons.push_back(MonD{bx[0], bx[1], bx[2], bx[3], bx[4], 0, bx[4], 0, cnt, off, out});
       off += cnt;
       ++k;
     }
@@ -1559,7 +1821,14 @@ static int prepare_common(const GdnTmParams* p, const GdnTmPoints* pts, const Gd
   if (!R.mons.empty())
     GDN_TRY_CUDA(cudaMemcpyAsync(ws + L.mons, R.mons.data(), R.mons.size() * sizeof(MonD),
                                  cudaMemcpyHostToDevice, stream));
+  return prepare_state(p, b, ws, R, stream);
+}
 
+template <typename T>
+static int prepare_state(const GdnTmParams* p, const GdnTmBuffers* b, char* ws, Run<T>& R,
+                         cudaStream_t stream) {
+  const Layout& L = R.L;
+  const int nx = p->nx, ny = p->ny, N = p->n_steps;
   // Clear the state that starts at zero: both field slots (ghost cells
   // included), padded ca/cb, both psi parities, the step counter.
   GDN_TRY_CUDA(cudaMemsetAsync(ws + L.state[0], 0, L.zero_end - L.state[0], stream));
@@ -1585,20 +1854,408 @@ static int finalize(const GdnTmParams* p, const GdnTmBuffers* b, const Run<T>& R
   const int eblocks = int(std::min<long long>(div_up((long long)nx * ny, 256), 148 * 8));
   tm_copy_out<T><<<eblocks, 256, 0, stream>>>(last, R.L.plane, nx, ny, R.L.ld,
                                               static_cast<T*>(b->ez), static_cast<T*>(b->hx),
-                                              static_cast<T*>(b->hy));
+                                              static_cast<T*>(b->hy), R.err);
   for (const MonD& m : R.mons) {
     const long long cnt = m.count * p->n_freq;
     const int blocks = int(std::min<long long>(div_up(cnt, 256), 148 * 8));
     if (p->dft_f64)
-      tm_dft_scale<double2><<<blocks, 256, 0, stream>>>(static_cast<double2*>(m.out), cnt, p->dt);
+      tm_dft_scale<double2><<<blocks, 256, 0, stream>>>(static_cast<double2*>(m.out), cnt, p->dt,
+                                                       R.err);
     else
-      tm_dft_scale<float2><<<blocks, 256, 0, stream>>>(static_cast<float2*>(m.out), cnt, p->dt);
+      tm_dft_scale<float2><<<blocks, 256, 0, stream>>>(static_cast<float2*>(m.out), cnt, p->dt,
+                                                      R.err);
   }
   if (p->record_energy && N > 0)
     tm_energy_finish<T><<<unsigned(div_up(N, 256)), 256, 0, stream>>>(
         R.eacc, static_cast<T*>(b->out_energy), N, p->dx * p->dy, p->mu0);
   count_launches(1 + R.mons.size() + (p->record_energy && N > 0 ? 1 : 0));
   GDN_TRY_CUDA(cudaGetLastError());
+  return GDN_OK;
+}
+
+
+// ---------------------------------------------------------------------------
+// Resident kernels: tables, launches
+// ---------------------------------------------------------------------------
+
+// Call f with the interior and general shapes of a kind of field type T.
+template <typename T, typename F>
+static int with_kind(int kind, F&& f) {
+  if constexpr (std::is_same<T, float>::value) {
+    switch (kind) {
+      case 0: return f(res::F32A{}, res::F32A{});
+      case 1: return f(res::F32B{}, res::F32A{});
+      case 2: return f(res::F32C{}, res::F32CG{});
+      case 3: return f(res::F32D{}, res::F32DG{});
+      default: return f(res::F32E{}, res::F32EG{});
+    }
+  } else {
+    switch (kind) {
+      case 0: return f(res::F64A{}, res::F64A{});
+      case 1: return f(res::F64B{}, res::F64A{});
+      default: return f(res::F64C{}, res::F64CG{});
+    }
+  }
+}
+
+// Bytes appended to a host image, 16-byte aligned; returns their offset.
+template <typename X>
+static size_t append(std::vector<char>& blob, const X* x, size_t n) {
+  const size_t at = (blob.size() + 15) / 16 * 16;
+  blob.resize(at + n * sizeof(X));
+  if (n) std::copy_n(reinterpret_cast<const char*>(x), n * sizeof(X), blob.data() + at);
+  return at;
+}
+
+// Monitors, rectangles and per-thread point lists of a run, in one upload.
+template <typename T>
+static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers* b,
+                       char* ws, Run<T>& R, cudaStream_t stream) {
+  const Layout& L = R.L;
+  const Plan& pl = L.plan;
+  Dev<T>& d = R.d;
+  const int nr = pl.n_rects;
+  std::vector<char> blob;
+  blob.reserve(L.blob_bytes);
+  char* const base = ws + L.blob;
+  auto dev = [&](size_t at) { return base + at; };
+
+  // Rectangles, general ones first (they take longest).
+  std::vector<res::RTile> tiles(nr);
+  for (const Region& g : pl.regions)
+    for (int r = 0; r < g.nr; ++r)
+      for (int q = 0; q < g.nc; ++q) {
+        const res::Rect x = rect_at(g, r, q);
+        const int idx = g.first + r * g.nc + q;
+        tiles[idx] = res::RTile{0, idx, -1, x.i0, x.j0, x.h, x.w, x.gen};
+      }
+
+  // Monitors and their parts per rectangle.
+  R.mons.clear();
+  {
+    void* const full_out[3] = {b->dft_ez, b->dft_hx, b->dft_hy};
+    const size_t csz = p->dft_f64 ? sizeof(double2) : sizeof(float2);
+    long long off = 0;
+    int k = 0;
+    for (const auto& bx : monitor_boxes(p, pts)) {
+      void* out = p->n_monitors == 0 ? full_out[k] : pts->monitors[k].out;
+      const int pitch = ring_pitch(bx[2], bx[4]);
+      const MonD m{bx[0], bx[1], bx[2], bx[3], bx[4], bx[2] % 4, pitch, 0, (long long)bx[3] * bx[4], off, out};
+      off += (long long)bx[3] * pitch;
+      R.mons.push_back(m);
+      GDN_TRY_CUDA(cudaMemsetAsync(out, 0, size_t(m.count) * p->n_freq * csz, stream));
+      ++k;
+    }
+  }
+  std::vector<int> moff(nr + 1, 0);
+  std::vector<MonW> mw(static_cast<size_t>(L.n_mw));
+  {
+    for (const MonD& m : R.mons)
+      rects_of(pl, m.lo0, m.lo0 + m.h, m.lo1, m.lo1 + m.w,
+               [&](const Region&, int, int, int idx) { ++moff[idx + 1]; });
+    for (int t = 0; t < nr; ++t) moff[t + 1] += moff[t];
+    if (moff[nr] != L.n_mw)
+      GDN_BAD_ARG("internal: %d monitor parts, layout sized for %lld", moff[nr], L.n_mw);
+    std::vector<int> at(moff.begin(), moff.end() - 1);
+    for (const MonD& m : R.mons)
+      rects_of(pl, m.lo0, m.lo0 + m.h, m.lo1, m.lo1 + m.w, [&](const Region& g, int r, int q, int idx) {
+        const res::Rect x = rect_at(g, r, q);
+        MonW e;
+        e.a0 = std::max(m.lo0, x.i0);
+        e.a1 = std::min(m.lo0 + m.h, x.i0 + x.h);
+        e.b0 = std::max(m.lo1, x.j0);
+        e.b1 = std::min(m.lo1 + m.w, x.j0 + x.w);
+        e.comp = m.comp;
+        e.w = m.pitch;
+        e.base = m.off + m.pad - m.lo1 - (long long)m.lo0 * m.pitch;
+        mw[at[idx]++] = e;
+      });
+  }
+
+  // Points: per rectangle the injections (ports first), per thread its entries
+  // in the order a step applies them. Records (ports' V and I, probes) belong
+  // to the owner; injections to every copy.
+  const int counts[5] = {p->n_ports, p->n_sources, p->n_mx, p->n_my, p->n_probes};
+  const int32_t* is[5] = {pts->port_i, pts->src_i, pts->mx_i, pts->my_i, pts->probe_i};
+  const int32_t* js[5] = {pts->port_j, pts->src_j, pts->mx_j, pts->my_j, pts->probe_j};
+  const int id0[4] = {p->n_sources + p->n_mx + p->n_my, 0, p->n_sources, p->n_sources + p->n_mx};
+  if (counts[0] > MAXP) {  // the tile kernels' limit, whatever the rectangles
+    const Bins bn = bin_tiles(counts[0], is[0], js[0], L, true);
+    if (bn.max_per_tile > MAXP)
+      GDN_BAD_ARG("%d port records fall in one tile (at most %d)", bn.max_per_tile, MAXP);
+  }
+  struct Copy {
+    int type, m, i, j, own;
+  };
+  std::vector<std::vector<Copy>> in(nr);
+  bool any = false;
+  for (int k = 0; k < 5; ++k)
+    for (int m = 0; m < counts[k]; ++m) {
+      const int i = is[k][m], j = js[k][m], halo = k < 4 ? res::TB : 0;
+      any = true;
+      rects_of(pl, i - halo, i + halo + 1, j - halo, j + halo + 1, [&](const Region& g, int r, int q, int idx) {
+        const res::Rect x = rect_at(g, r, q);
+        const int own = i >= x.i0 && i < x.i0 + x.h && j >= x.j0 && j < x.j0 + x.w;
+        in[idx].push_back(Copy{k, m, i, j, own});
+      });
+    }
+  std::vector<res::RHdr> hdr;
+  std::vector<int> vl_off(nr + 1, 0), vl, pts_off(1, 0);
+  std::vector<res::RPt> ents;
+  if (any) {
+    const ShapeInfo main = kind_shape(sizeof(T), L.kind, false);
+    std::vector<int> cnt(size_t(main.nt) * 4);
+    const int staged = 4096 / int(sizeof(T)) / res::TB;  // values a rectangle stages
+    int slots = 0;
+    for (int t = 0; t < nr; ++t) {
+      if (!in[t].empty()) {
+        res::RTile& x = tiles[t];
+        x.slot = slots++;
+        const ShapeInfo s = kind_shape(sizeof(T), L.kind, x.gen != 0);
+        const int V = s.ew / 32, RR = s.eh / (s.nt / 32);
+        auto place = [&](const Copy& q, int* reg) {
+          const int r = q.i - x.i0 + res::TB, c = q.j - x.j0 + res::TB;
+          *reg = r % RR * V + c % V;
+          return r / RR * 32 + c / V;
+        };
+        // Classes per thread: 0 Mx/My, 1 Jz, 2 ports, 3 probes.
+        const int cls_of[5] = {2, 1, 0, 0, 3};
+        std::fill(cnt.begin(), cnt.end(), 0);
+        int reg;
+        for (const Copy& q : in[t]) ++cnt[size_t(place(q, &reg)) * 4 + cls_of[q.type]];
+        const int e0 = int(ents.size());
+        int at = e0;
+        ents.resize(ents.size() + in[t].size());
+        for (int th = 0; th < s.nt; ++th) {
+          int* const n = &cnt[size_t(th) * 4];
+          hdr.push_back(res::RHdr{at - e0, unsigned(n[0]) | unsigned(n[1]) << 16,
+                                  unsigned(n[2]) | unsigned(n[3]) << 16, 0, 0, 0, 0, 0, 0});
+          for (int k = 0; k < 4; ++k) {
+            const int here = n[k];
+            n[k] = at;
+            at += here;
+          }
+        }
+        // Entries in point order; injected values are numbered below.
+        for (const Copy& q : in[t]) {
+          const int th = place(q, &reg);
+          const int kind = q.type == 0 ? q.own : q.type == 3 ? 1 : 0;
+          res::RPt e{q.m, unsigned(reg) | unsigned(kind) << 8};
+          if (q.type == 1) e.m = id0[1] + q.m;
+          if (q.type == 2 || q.type == 3) e.m = id0[q.type] + q.m;
+          ents[cnt[size_t(th) * 4 + cls_of[q.type]]++] = e;
+        }
+        // Values: ports in port order, then every thread's magnetic and electric
+        // currents, by register where no register has two.
+        int val = 0;
+        for (const Copy& q : in[t])
+          if (q.type == 0) {
+            vl.push_back(id0[0] + q.m);
+            ++val;
+          }
+        const int v0 = int(vl.size()) - val;  // values of this rectangle start here
+        int port = 0;
+        std::vector<std::pair<int, int>> port_val;  // (m, value)
+        for (const Copy& q : in[t])
+          if (q.type == 0) port_val.push_back({q.m, port++});
+        res::RHdr* const h0 = &hdr[hdr.size() - size_t(s.nt)];
+        for (int th = 0; th < s.nt; ++th) {
+          res::RHdr& h = h0[th];
+          res::RPt* x0 = ents.data() + e0 + h.first;
+          const int n_mag = int(h.n01 & 0xffff), n_jz = int(h.n01 >> 16), n_port = int(h.n23 & 0xffff);
+          for (int cls = 0; cls < 2; ++cls) {
+            res::RPt* const a = cls == 0 ? x0 : x0 + n_mag;
+            const int n = cls == 0 ? n_mag : n_jz;
+            unsigned mask[2] = {0, 0};
+            bool once = n > 0;
+            for (int q = 0; q < n; ++q) {
+              unsigned& mk = mask[cls == 0 ? a[q].kind() : 0];
+              once = once && a[q].reg() < 32 && !(mk >> a[q].reg() & 1);
+              if (a[q].reg() < 32) mk |= 1u << a[q].reg();
+            }
+            if (once)
+              std::sort(a, a + n, [](const res::RPt& x, const res::RPt& y) {
+                return std::make_pair(x.kind(), x.reg()) < std::make_pair(y.kind(), y.reg());
+              });
+            const int first = int(vl.size()) - v0;
+            for (int q = 0; q < n; ++q) {
+              a[q].w |= unsigned(int(vl.size()) - v0) << 10;
+              vl.push_back(a[q].m);
+            }
+            if (once && first + n <= staged) {
+              h.dense |= 1u << cls;
+              if (cls == 0) {
+                h.m_hx = mask[0];
+                h.m_hy = mask[1];
+                h.v_h = static_cast<unsigned short>(first);
+              } else {
+                h.m_e = mask[0];
+                h.v_e = static_cast<unsigned short>(first);
+              }
+            }
+          }
+          for (int q = 0; q < n_port; ++q) {
+            res::RPt& e = x0[n_mag + n_jz + q];
+            for (const auto& pv : port_val)
+              if (pv.first == e.m) e.w |= unsigned(pv.second) << 10;
+          }
+        }
+      }
+      vl_off[t + 1] = int(vl.size());
+      if (!in[t].empty()) pts_off.push_back(int(ents.size()));
+    }
+  }
+  R.rtiles = std::move(tiles);
+  R.rsmem = pl.smem;
+
+  res::RDev<T>& rd = R.rd;
+  const size_t a_rd = append(blob, &rd, 1), a_tiles = append(blob, R.rtiles.data(), R.rtiles.size());
+  d.n_mons = int(R.mons.size());
+  d.mons = reinterpret_cast<const MonD*>(dev(append(blob, R.mons.data(), R.mons.size())));
+  d.mw_off = reinterpret_cast<const int*>(dev(append(blob, moff.data(), moff.size())));
+  d.mw = reinterpret_cast<const MonW*>(dev(append(blob, mw.data(), mw.size())));
+  rd.vl_off = nullptr;
+  if (any) rd.vl_off = reinterpret_cast<const int*>(dev(append(blob, vl_off.data(), vl_off.size())));
+  rd.hdr = reinterpret_cast<const res::RHdr*>(dev(append(blob, hdr.data(), hdr.size())));
+  rd.pts_off = reinterpret_cast<const int*>(dev(append(blob, pts_off.data(), pts_off.size())));
+  rd.pts = reinterpret_cast<const res::RPt*>(dev(append(blob, ents.data(), ents.size())));
+  rd.vl = reinterpret_cast<const int*>(dev(append(blob, vl.data(), vl.size())));
+  rd.xch = reinterpret_cast<uint4*>(ws + L.xch);
+  rd.pv = reinterpret_cast<const T*>(ws + L.pv);
+  rd.n_inj = int(injections(p));
+  rd.dft_f64 = p->dft_f64 != 0;
+  rd.d = d;
+  std::copy_n(reinterpret_cast<const char*>(&rd), sizeof(rd), blob.data() + a_rd);
+  if (blob.size() > L.blob_bytes)
+    GDN_BAD_ARG("internal: %zu bytes of tables, layout sized for %zu", blob.size(), L.blob_bytes);
+  // Pageable: staged when the call returns, so the image may go away.
+  GDN_TRY_CUDA(cudaMemcpyAsync(base, blob.data(), blob.size(), cudaMemcpyHostToDevice, stream));
+  R.d_rd = reinterpret_cast<const res::RDev<T>*>(base + a_rd);
+  R.d_rtiles = reinterpret_cast<const res::RTile*>(base + a_tiles);
+  R.err = reinterpret_cast<int*>(ws + L.err);
+  return GDN_OK;
+}
+
+// Problems advanced together by resident launches (a single run: one).
+template <typename T>
+struct Wave {
+  const res::RDev<T>* devs = nullptr;
+  const res::RTile* tiles = nullptr;
+  int* err = nullptr;
+  int n_prob = 0, n_tiles = 0, kind = 0, seg = 0, n_steps = 0, kmax = 0;
+  long long inj_max = 0, mon_max = 0;
+  bool f32 = false, f64 = false;  // DFT accumulator types present
+  size_t smem = 0;
+
+  void add(const GdnTmParams* p, const Run<T>& R) {
+    ++n_prob;
+    n_tiles += int(R.rtiles.size());
+    n_steps = std::max(n_steps, p->n_steps);
+    kmax = std::max(kmax, p->n_freq);
+    inj_max = std::max(inj_max, injections(p));
+    smem = std::max(smem, R.rsmem);
+    if (!R.mons.empty()) {
+      mon_max = std::max(mon_max, R.L.mon_cells);
+      (p->dft_f64 ? f64 : f32) = true;
+    }
+  }
+};
+
+// One cooperative launch. Tiles of two such launches wait only for their own,
+// but each needs all of its tiles on the device: launches of this process on
+// one device follow one another.
+template <class S, class S2>
+static int launch_coop(const res::RArgs<typename S::T>& a, int n_tiles, size_t smem,
+                       cudaStream_t stream) {
+  static std::mutex& mu = coop_mutex();
+  int dev = 0;
+  GDN_TRY_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  cudaEvent_t ev = coop_event(dev);
+  if (!ev) GDN_BAD_ARG("no event for this device");
+  GDN_TRY_CUDA(cudaStreamWaitEvent(stream, ev, 0));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(n_tiles));
+  cfg.blockDim = dim3(S::NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  GDN_TRY_CUDA(cudaLaunchKernelEx(&cfg, res::tm_res<S, S2>, a));
+  GDN_TRY_CUDA(cudaEventRecord(ev, stream));
+  return GDN_OK;
+}
+
+template <typename T, typename A, int KM, int NC>
+static void launch_seg_fold_nc(const Wave<T>& w, int seg0, cudaStream_t s) {
+  const dim3 grid(unsigned(div_up(w.mon_max, 256 * NC)), unsigned(w.n_prob));
+  const size_t sm = size_t(4) * res::FOLD * w.kmax * sizeof(A);
+  res::tm_seg_fold<T, A, KM, NC><<<grid, 256, sm, s>>>(w.devs, seg0, w.seg);
+}
+
+// Cells per thread: as many as the accumulators leave registers for, and one
+// where few cells would leave SMs idle.
+template <typename T, typename A>
+static void launch_seg_fold(const Wave<T>& w, int seg0, cudaStream_t s) {
+  constexpr bool wide = sizeof(A) == 8;
+  const bool few = w.mon_max < 148 * 1024;
+  if (w.kmax <= 4)
+    few ? launch_seg_fold_nc<T, A, 4, 1>(w, seg0, s) : launch_seg_fold_nc<T, A, 4, wide ? 1 : 4>(w, seg0, s);
+  else if (w.kmax <= 8)
+    few ? launch_seg_fold_nc<T, A, 8, 1>(w, seg0, s) : launch_seg_fold_nc<T, A, 8, wide ? 1 : 2>(w, seg0, s);
+  else
+    launch_seg_fold_nc<T, A, KMAX, 1>(w, seg0, s);
+}
+
+// All time steps of a wave: per segment the value table, the tiles (one
+// cooperative launch when they all fit, else one launch per block) and the
+// DFT sums.
+template <typename T>
+static int run_wave(const Wave<T>& w, cudaStream_t stream) {
+  return with_kind<T>(w.kind, [&](auto sh, auto sh2) -> int {
+    using S = decltype(sh);
+    using S2 = decltype(sh2);
+    int st;
+    GDN_TRY_CUDA(cudaFuncSetAttribute(res::tm_res<S, S2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      220 * 1024));
+    uint64_t k = 0;
+    for (int seg0 = 0; seg0 < w.n_steps; seg0 += w.seg) {
+      const int cnt = std::min(w.seg, w.n_steps - seg0);
+      if (w.inj_max > 0) {
+        res::tm_values<T><<<dim3(unsigned(div_up(w.inj_max, 128)), unsigned(div_up(cnt, res::FOLD)),
+                                 unsigned(w.n_prob)), 128, 0, stream>>>(w.devs, seg0, w.seg);
+        ++k;
+      }
+      const int b0 = seg0 / res::TB, b1 = int(div_up(seg0 + cnt, res::TB));
+      res::RArgs<T> a{w.devs, w.tiles, w.err, b0, b1, seg0};
+      if ((st = launch_coop<S, S2>(a, w.n_tiles, w.smem, stream))) return st;
+      ++k;
+      if (w.f64) launch_seg_fold<T, double>(w, seg0, stream);
+      if (w.f32) launch_seg_fold<T, float>(w, seg0, stream);
+      k += int(w.f64) + int(w.f32);
+    }
+    const cudaError_t le = cudaGetLastError();
+    if (le != cudaSuccess) {
+      set_error("launch failed: %s", cudaGetErrorString(le));
+      return GDN_ERR_CUDA;
+    }
+    count_launches(k);
+    return GDN_OK;
+  });
+}
+
+// A stream capture cannot hold a run: its tables come from host memory that
+// is gone when the call returns.
+static int refuse_capture(cudaStream_t stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  GDN_TRY_CUDA(cudaStreamIsCapturing(stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) {
+    set_error("graph launch failed: operation not permitted when stream is capturing");
+    return GDN_ERR_CUDA;
+  }
   return GDN_OK;
 }
 
@@ -1610,10 +2267,20 @@ static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers*
   if ((st = set_kernel_attributes<T>())) return st;
   Run<T> R;
   R.L = make_layout(p, pts, sizeof(T));
+  if (R.L.res && (st = refuse_capture(stream))) return st;
   char* ws = static_cast<char*>(b->workspace);
   bool own = false;
+  // Scratch that holds the tile kernels' layout only is enough for them.
+  if (ws && R.L.res && b->workspace_bytes < R.L.total)
+    R.L = make_layout(p, pts, sizeof(T), 0, -1, false);
   if (!ws) {
-    GDN_TRY_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&ws), R.L.total, stream));
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ws), R.L.total, stream);
+    if (e == cudaErrorMemoryAllocation && R.L.res) {
+      cudaGetLastError();
+      R.L = make_layout(p, pts, sizeof(T), 0, -1, false);
+      e = cudaMallocAsync(reinterpret_cast<void**>(&ws), R.L.total, stream);
+    }
+    GDN_TRY_CUDA(e);
     own = true;
   } else if (b->workspace_bytes < R.L.total) {
     GDN_BAD_ARG("workspace too small: %zu < %zu bytes", b->workspace_bytes, R.L.total);
@@ -1627,6 +2294,19 @@ static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers*
     }
   } guard{ws, own, stream};
   if ((st = prepare(p, pts, b, ws, R, stream))) return st;
+  if (R.L.res) {
+    Wave<T> w;
+    w.add(p, R);
+    w.devs = R.d_rd;
+    w.tiles = R.d_rtiles;
+    w.err = R.err;
+    w.kind = R.L.kind;
+    w.seg = R.L.seg;
+    LoopTimer timer(stream, double(p->nx) * p->ny * p->n_steps, div_up(p->n_steps, res::TB));
+    st = run_wave(w, stream);
+    timer.stop(st == GDN_OK);
+    return st ? st : finalize(p, b, R, stream);
+  }
 
   // Capture one chunk of `cnt` steps as a graph; the general and interior
   // tile launches of each block become parallel branches.
@@ -1751,7 +2431,7 @@ static int run_batch_f32(const GdnTmProblem* probs, int n, int cfg, cudaStream_t
   std::vector<Run<T>> R(n);
   int ring = 1 << 30;
   for (int q = 0; q < n; ++q) {
-    R[q].L = make_layout(probs[q].params, probs[q].points, sizeof(T), 0, which);
+    R[q].L = make_layout(probs[q].params, probs[q].points, sizeof(T), 0, which, false);
     ring = std::min(ring, R[q].L.R);
   }
   const int tb = kCfgF32[which].tb;
@@ -1761,7 +2441,7 @@ static int run_batch_f32(const GdnTmProblem* probs, int n, int cfg, cudaStream_t
   size_t own_bytes = 0;
   for (int q = 0; q < n; ++q) {
     if (R[q].L.R != ring)
-      R[q].L = make_layout(probs[q].params, probs[q].points, sizeof(T), ring, which);
+      R[q].L = make_layout(probs[q].params, probs[q].points, sizeof(T), ring, which, false);
     const GdnTmBuffers* b = probs[q].buffers;
     if (b->workspace) {
       if (b->workspace_bytes < R[q].L.total)
@@ -1907,7 +2587,10 @@ extern "C" int gdn_tm_workspace_size(const GdnTmParams* p, const GdnTmPoints* pt
     gdn::set_error("monitor list is null");
     return GDN_ERR_BAD_ARG;
   }
-  *bytes = gdn::tm2d::make_layout(p, pts, f64 ? sizeof(double) : sizeof(float)).total;
+  // A batch runs the tile kernels on the same scratch, a single run may not.
+  const size_t esize = f64 ? sizeof(double) : sizeof(float);
+  *bytes = std::max(gdn::tm2d::make_layout(p, pts, esize).total,
+                    gdn::tm2d::make_layout(p, pts, esize, 0, -1, false).total);
   return GDN_OK;
 }
 
@@ -1969,10 +2652,10 @@ static int run_noalloc_f32(const GdnTmParams* p, const GdnTmPoints* pts, const G
   if ((st = set_kernel_attributes<T>())) return st;
   // Largest monitor-ring length (a multiple of TB) whose layout fits.
   Run<T> R;
-  R.L = make_layout(p, pts, sizeof(T));
+  R.L = make_layout(p, pts, sizeof(T), 0, -1, false);
   const int tb = R.L.cfg.tb;
   for (int r = R.L.R; r > tb && R.L.total > kStaticScratchBytes; r -= tb)
-    R.L = make_layout(p, pts, sizeof(T), r - tb);
+    R.L = make_layout(p, pts, sizeof(T), r - tb, -1, false);
   if (R.L.total > kStaticScratchBytes)
     GDN_BAD_ARG("this run needs %zu bytes of scratch; the static scratch of "
                 "gdn_tm_run_noalloc_f32 holds %zu bytes (use gdn_tm_run_f32)",
