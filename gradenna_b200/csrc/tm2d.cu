@@ -2270,8 +2270,10 @@ static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers*
   if (R.L.res && (st = refuse_capture(stream))) return st;
   char* ws = static_cast<char*>(b->workspace);
   bool own = false;
-  // Scratch that holds the tile kernels' layout only is enough for them.
-  if (ws && R.L.res && b->workspace_bytes < R.L.total)
+  // Scratch that holds the tile kernels' layout only, or off the 16-byte
+  // boundaries that the exchanged words need, is enough for them.
+  if (ws && R.L.res &&
+      (b->workspace_bytes < R.L.total || reinterpret_cast<uintptr_t>(ws) % 16))
     R.L = make_layout(p, pts, sizeof(T), 0, -1, false);
   if (!ws) {
     cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ws), R.L.total, stream);
