@@ -9,16 +9,28 @@
 //
 // B200 design: two kernels per step updating in place (the H kernel reads
 // only E and the E kernel only H, so no CTA ever reads a value another CTA is
-// writing). A CTA covers an 8 x 32 (j, k) tile with k contiguous, so every
-// field access is a coalesced row, and walks 8 consecutive i-planes. Each
-// thread loads all operands of its cell before updating it. CPML psi lives
-// in full padded volumes (zero outside the slabs) indexed like the fields;
-// only slab cells touch them, on per-thread slab flags. Point work (sources,
-// the port, probes) is binned by plane box on the host and applied by the
-// owning CTA after its sweep; per plane-box flags keep the other boxes on the
-// bare stencil. The running DFT uses the monitor ring of the 2D path: after
-// each half step a gather kernel copies the monitored cells to ring slot
-// n % R, and one fold kernel per R steps adds sum_t ph[t,k] x_t to the
+// writing). A thread owns 16 bytes of cells along k (four float, two double) of
+// a row, a CTA 128 such vectors that follow one another over a plane's rows (no
+// lane is lost to nz), on two i-planes: the curl, update and padding work is
+// paid per vector load, the z slabs of all cells of a vector in one pass. All
+// operands of a plane, psi included, are loaded before the first use. CPML psi
+// lives in full padded volumes (zero outside the slabs) indexed like the
+// fields; only slab cells touch them. ca, cb are laid out like the fields when a
+// run starts, the CPML coefficients as tables by node.
+//   What bounds it: the L2 round trip of a plane's loads with 16 warps an SM
+// (ncu at 160 x 160 x 64 f32: issue 12 %, long-scoreboard stalls 70 %, H 18 us
+// and E 21 us a step; their 160 MB at L2 rates would take about 20 us a step).
+// One cell a thread, 8 x 32 boxes, was issue bound: 252 (H) and 300 (E) warp
+// instructions per 32 cells. More warps with fewer registers lose to spills (5
+// CTAs an SM: 390 ms for the run of 3 below, 6: 435), 8-byte vectors with 6: 317.
+//   Measured, whole calls:  97 x 83 x 61 f32, 600 steps            13.6 -> 10.6 ms
+//                           64 x 64 x 48 f64, 400 steps             8.5 -> 7.2 ms
+//                           160 x 160 x 64 f32 gradient, 2 x 3000   344 -> 300 ms
+//   Point work (sources near probes, the port, probes) is binned by plane and
+// CTA on the host and applied by the owner after its sweep. The running DFT uses
+// the monitor ring of the 2D path: after each half step a gather kernel copies
+// the monitored cells to ring slot n % R, and one fold kernel per R steps adds
+// sum_t ph[t,k] x_t to the
 // accumulators. One chunk of R steps is captured as a CUDA graph and
 // replayed; kernels read the absolute step from a counter.
 #include <algorithm>
@@ -30,8 +42,8 @@
 namespace gdn {
 namespace yee3d {
 
-constexpr int BK = 32, BJ = 8;  // CTA box along k and j (one i-plane)
-constexpr int NT = BK * BJ;
+constexpr int NT = 128;           // threads of a step kernel's CTA
+constexpr int BK = 32, BJ = 8;    // boxes of the CPML rounding classes (k, j)
 constexpr int KMAX = 16;
 constexpr int NC = 6;  // components: ex ey ez hx hy hz
 
@@ -56,12 +68,15 @@ struct Mon3 {
 
 template <typename T>
 struct Dev3 {
-  int nx, ny, nz, npml, n_steps, n_freq, R, gj, gk;  // gj, gk: CTA grid along j, k
+  int nx, ny, nz, npml, n_steps, n_freq, R, tw;  // tw: vectors of V cells a row
   int sy, sz;          // padded strides: cell (i,j,k) at ((i+1)*sy + (j+1))*sz + (k+1)
   long long vol;       // elements per padded volume
   T* f[NC];            // fields
   T* psi;              // 12 padded volumes (see psi_* constants)
   const T *ca, *cb, *eps;  // caller (nx, ny, nz)
+  const T *cap, *cbp;      // ca, cb laid out like the fields, or null
+  const T* tab;            // CPML b, c, 1/kappa by node: [E, H][axis][3][ts]
+  int ts;
   const T *ik_e[3], *ik_h[3];
   const T *be_lo[3], *ce_lo[3], *be_hi[3], *ce_hi[3];
   const T *bh_lo[3], *ch_lo[3], *bh_hi[3], *ch_hi[3];
@@ -94,7 +109,7 @@ struct Dev3 {
   const unsigned* gsrc;
   const long long* gsrc64;
   long long gcells[2];
-  const unsigned char* cls;  // per plane-box work flags (F_*)
+  const unsigned char* cls;  // [plane][column block]: F_EPTS or 0
   T* cwv;                // CW source values of the chunk: [sub][cw_off[type] + m]
   long long cw_total, cw_off[6];
   const int* step_base;
@@ -218,12 +233,8 @@ __global__ void __launch_bounds__(256) yee_gather(Dev3<T> d, int sub, int side) 
   d.mring[(long long)(n % d.R) * d.mon_cells + at_r] = d.f[0][src];
 }
 
-// Per plane-box flags (bit set = the box needs that work), computed on the
-// host so that most boxes run the bare stencil with no per-thread checks.
-enum : unsigned char { F_HPTS = 1, F_EPTS = 2, F_CPML = 8 };
-
-// A CTA walks `ni` consecutive i-planes of its (j, k) tile (chosen on the
-// host, planes_per_cta).
+// Flag of a (plane, column block): its CTA applies points or the port there.
+constexpr unsigned char F_EPTS = 2;
 
 // CPML coefficients of sample s of axis ax (E-type: the ns = n-2 samples
 // of the PEC interior; H-type: the ns = n-1 half samples). Returns whether
@@ -252,273 +263,445 @@ __device__ __forceinline__ bool slab_coef(const Dev3<T>& d, int ax, int s, int n
   return false;
 }
 
-// One axis' CPML state of a thread: whether its sample is in a slab and the
-// coefficients there.
+// ---- vectors of V cells along k ----
+//
+// A row of a padded volume starts with the cell k = -1 on a 16-byte boundary,
+// so vector t of a row holds the cells V t - 1 .. V t + V - 2.
+
+template <typename T>
+struct alignas(16) Vec {
+  static constexpr int V = 16 / int(sizeof(T));
+  T v[V];
+  __device__ __forceinline__ T& operator[](int x) { return v[x]; }
+  __device__ __forceinline__ const T& operator[](int x) const { return v[x]; }
+};
+template <typename T>
+__device__ __forceinline__ Vec<T> ldv(const T* p) {
+  return *reinterpret_cast<const Vec<T>*>(p);
+}
+template <typename T>
+__device__ __forceinline__ void stv(T* p, const Vec<T>& v) {
+  *reinterpret_cast<Vec<T>*>(p) = v;
+}
+
+// Roundings are written out: a result must not depend on how a kernel was cut
+// or compiled, and boxes of the two classes below round X differently.
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float sub_(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double sub_(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// The bit x of a mask for cells x = 0 .. V - 1 with lo <= k0 + x < hi.
+template <int V>
+__device__ __forceinline__ unsigned range_mask(int k0, int lo, int hi) {
+  unsigned m = 0;
+#pragma unroll
+  for (int x = 0; x < V; ++x) m |= unsigned(k0 + x >= lo && k0 + x < hi) << x;
+  return m;
+}
+
+// Whether cells [lo, hi) of an axis of n nodes reach a CPML slab (of either
+// field type, one cell of margin). A plane box of BJ x BK cells that does along
+// any axis is of the general class.
+__device__ __forceinline__ bool near_slab(int m, int lo, int hi, int n) {
+  return m > 0 && (lo <= m + 1 || hi - 1 >= n - 2 - m);
+}
+
+// Whether CPML sample s of ns lies in a slab of m cells.
+__device__ __forceinline__ bool in_slab(int m, int s, int ns) {
+  return (s >= 0 && s < m) || (s >= ns - m && s < ns);
+}
+
+// Tables of the CPML coefficients by node p = -1 .. ts - 2 (E-type samples are
+// node - 1): no slab test stands before their loads.
+template <typename T>
+__global__ void yee_tables(Dev3<T> d, T* tab) {
+  const int p = int(blockIdx.x * blockDim.x + threadIdx.x) - 1, ax = blockIdx.y;
+  if (p + 1 >= d.ts) return;
+  const int n = ax == 0 ? d.nx : (ax == 1 ? d.ny : d.nz);
+  T b, c, ik;
+  slab_coef<T, true>(d, ax, p - 1, n - 2, b, c, ik);
+  T* o = tab + 3 * ax * d.ts + p + 1;
+  o[0] = b;
+  o[d.ts] = c;
+  o[2 * d.ts] = ik;
+  slab_coef<T, false>(d, ax, p, n - 1, b, c, ik);
+  o += 9 * d.ts;
+  o[0] = b;
+  o[d.ts] = c;
+  o[2 * d.ts] = ik;
+}
+
+// CPML coefficients of one sample, and of a thread's cells along z.
 template <typename T>
 struct Ax {
-  bool on;
   T b, c, ik;
 };
-
-// psi <- b psi + c diff; the term diff/kappa + psi (cpml.py:120-158).
 template <typename T>
-__device__ __forceinline__ T psi_term(const Ax<T>& a, T diff, T& psi) {
-  psi = a.b * psi + a.c * diff;
-  return diff * a.ik + psi;
+struct Az {
+  Vec<T> b, c, ik;
+};
+template <typename T, bool E>
+__device__ __forceinline__ Ax<T> coef_at(const Dev3<T>& d, int ax, int p) {
+  const T* t = d.tab + ((E ? 0 : 9) + 3 * ax) * d.ts + p + 1;
+  return Ax<T>{t[0], t[d.ts], t[2 * d.ts]};
+}
+template <typename T, bool E>
+__device__ __forceinline__ Az<T> coef_z(const Dev3<T>& d, int k0) {
+  const T* t = d.tab + ((E ? 0 : 9) + 6) * d.ts + k0 + 1;
+  return Az<T>{ldv(t), ldv(t + d.ts), ldv(t + 2 * d.ts)};
+}
+template <int V>
+__device__ __forceinline__ unsigned slab_mask(int m, int s0, int ns) {
+  unsigned r = 0;
+#pragma unroll
+  for (int x = 0; x < V; ++x) r |= unsigned(in_slab(m, s0 + x, ns)) << x;
+  return r;
+}
+
+// A term's psi; X of a cell whose box reaches no slab; a field E.
+template <typename T>
+__device__ __forceinline__ T psi_next(T b, T psi, T c, T diff) {
+  return fma_(c, diff, mul_(b, psi));
+}
+template <typename T>
+__device__ __forceinline__ T x_bare(T d1, T i1, T d2, T i2) {
+  return fma_(d1, i1, -mul_(d2, i2));
+}
+template <typename T>
+__device__ __forceinline__ T e_next(T ca, T e, T cb, T x) {
+  return fma_(ca, e, mul_(cb, x));
+}
+
+// Terms t[x] = difference times 1/d of one curl part, with its CPML stretch in
+// the cells `on` (coefficients by cell or one for all).
+template <typename T>
+__device__ __forceinline__ void stretch(const Ax<T>& a, unsigned on, Vec<T>& q, Vec<T>& t) {
+  if (!on) return;
+#pragma unroll
+  for (int x = 0; x < Vec<T>::V; ++x)
+    if (on >> x & 1) {
+      q[x] = psi_next(a.b, q[x], a.c, t[x]);
+      t[x] = fma_(t[x], a.ik, q[x]);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void stretch(const Az<T>& a, unsigned on, Vec<T>& q, Vec<T>& t) {
+  if (!on) return;
+#pragma unroll
+  for (int x = 0; x < Vec<T>::V; ++x)
+    if (on >> x & 1) {
+      q[x] = psi_next(a.b[x], q[x], a.c[x], t[x]);
+      t[x] = fma_(t[x], a.ik[x], q[x]);
+    }
+}
+
+template <typename T>
+struct Thread3 {
+  static constexpr int V = Vec<T>::V;
+  int j, k0, c;      // row, first cell, offset of the first cell in plane i0
+  bool live;
+  unsigned gen;      // cells whose box reaches a y or z slab
+};
+template <typename T>
+__device__ __forceinline__ Thread3<T> locate(const Dev3<T>& d, int i0) {
+  constexpr int V = Vec<T>::V;
+  Thread3<T> t;
+  const int q = int(blockIdx.x) * NT + int(threadIdx.x);
+  t.j = q / d.tw;
+  const int v = q - t.j * d.tw;
+  t.live = t.j < d.ny;
+  t.k0 = V * v - 1;
+  t.c = ((i0 + 1) * d.sy + (t.j + 1)) * d.sz + V * v;
+  const int jb = t.j / BJ * BJ, ka = max(t.k0, 0) / BK * BK, kb = (t.k0 + 1) / BK * BK;
+  const bool gj = near_slab(d.npml, jb, min(d.ny, jb + BJ), d.ny);
+  const bool ga = near_slab(d.npml, ka, min(d.nz, ka + BK), d.nz);
+  const bool gb = near_slab(d.npml, kb, min(d.nz, kb + BK), d.nz);
+  constexpr unsigned ALL = (1u << V) - 1;
+  t.gen = gj ? ALL : ((ga ? 1u : 0u) | (gb ? ALL - 1 : 0u));
+  return t;
+}
+
+// ca, cb laid out like the fields (zero in the padding).
+template <typename T>
+__global__ void yee_pad_coef(Dev3<T> d, T* cap, T* cbp) {
+  const int ny = d.ny, nz = d.nz;
+  const long long total = (long long)d.nx * ny * nz;
+  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
+       g += (long long)gridDim.x * blockDim.x) {
+    const int i = int(g / ((long long)ny * nz));
+    const int rem = int(g - (long long)i * ny * nz);
+    const int j = rem / nz, k = rem - j * nz;
+    const long long c = at(d, i, j, k);
+    cap[c] = d.ca[g];
+    cbp[c] = d.cb[g];
+  }
 }
 
 // ---------------------------------------------------------------------------
-// H update: E^n -> H^{n+1/2} (fdtd3d.py:564-588) + Mx/My/Mz + H monitors.
-// A CTA covers a BJ x BK tile of NI consecutive i-planes.
+// H update: E^n -> H^{n+1/2} (fdtd3d.py:564-588). A CTA covers NT vectors of a
+// plane's rows and `ni` consecutive planes.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3) yee_h(Dev3<T> d, int sub, int ni) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, int ni) {
+  constexpr int V = Vec<T>::V;
+  constexpr unsigned ALL = (1u << V) - 1;
   dependent_launch_gate();
-  const int n = *d.step_base + sub;
-  const int k = blockIdx.x * BK + threadIdx.x;
-  const int j = blockIdx.y * BJ + threadIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  const bool live = j < ny && k < nz;
-  const int tid = threadIdx.y * BK + threadIdx.x;
-  const int i0 = int(blockIdx.z) * ni, i1 = min(nx, i0 + ni);
+  const int i0 = int(blockIdx.y) * ni, i1 = min(nx, i0 + ni);
+  const Thread3<T> th = locate(d, i0);
+  if (!th.live) return;
   // 32-bit cell offsets (a padded volume holds fewer than 2^31 cells).
   const int di = d.sy * d.sz, dj = d.sz;
-  int c = ((i0 + 1) * d.sy + (j + 1)) * d.sz + (k + 1);
+  int c = th.c;
   const T* __restrict__ ex = d.f[0];
   const T* __restrict__ ey = d.f[1];
   const T* __restrict__ ez = d.f[2];
   T *hx = d.f[3], *hy = d.f[4], *hz = d.f[5];
-  T *pxz = d.psi + P_HXZ * d.vol, *pxy = d.psi + P_HXY * d.vol, *pyx = d.psi + P_HYX * d.vol,
-    *pyz = d.psi + P_HYZ * d.vol, *pzy = d.psi + P_HZY * d.vol, *pzx = d.psi + P_HZX * d.vol;
   const T dt_mu = d.dt_mu, idx = d.inv_d[0], idy = d.inv_d[1], idz = d.inv_d[2];
   // This thread's y and z CPML samples (H-type) are fixed over the planes.
-  Ax<T> ay, az;
-  ay.on = slab_coef<T, false>(d, 1, j, ny - 1, ay.b, ay.c, ay.ik);
-  az.on = slab_coef<T, false>(d, 2, k, nz - 1, az.b, az.c, az.ik);
-  const bool vx = j < ny - 1 && k < nz - 1, kin = k < nz - 1, jin = j < ny - 1;
+  const Ax<T> ay = coef_at<T, false>(d, 1, th.j);
+  const Az<T> az = coef_z<T, false>(d, th.k0);
+  const bool yon = in_slab(d.npml, th.j, ny - 1);
+  const unsigned zon = slab_mask<V>(d.npml, th.k0, nz - 1);
+  const bool jin = th.j < ny - 1;
+  const unsigned kin = range_mask<V>(th.k0, 0, nz - 1), kall = range_mask<V>(th.k0, 0, nz);
   // Ey and Ez of plane i + 1 become plane i + 1's own values next iteration.
-  T ey0 = T(0), ez0 = T(0);
-  if (live) {
-    ey0 = ey[c];
-    ez0 = ez[c];
-  }
+  Vec<T> ey0 = ldv(ey + c), ez0 = ldv(ez + c);
   for (int i = i0; i < i1; ++i, c += di) {
-    const int cta = (i * d.gj + blockIdx.y) * d.gk + blockIdx.x;
-    const unsigned fl = d.cls[cta];
-    if (live && !(fl & F_CPML)) {
-      // No slab within reach of this plane box: the bare update.
-      const T ex0 = ex[c];
-      const T eyk = ey[c + 1], ezj = ez[c + dj], ezi = ez[c + di];
-      const T exk = ex[c + 1], exj = ex[c + dj], eyi = ey[c + di];
-      const T hx0 = hx[c], hy0 = hy[c], hz0 = hz[c];
-      const bool vy = i < nx - 1 && kin, vz = i < nx - 1 && jin;
-      if (vx) hx[c] = hx0 + dt_mu * ((eyk - ey0) * idz - (ezj - ez0) * idy);
-      if (vy) hy[c] = hy0 + dt_mu * ((ezi - ez0) * idx - (exk - ex0) * idz);
-      if (vz) hz[c] = hz0 + dt_mu * ((exj - ex0) * idy - (eyi - ey0) * idx);
-      ey0 = eyi;
-      ez0 = ezi;
-    } else if (live) {
-      Ax<T> ax;
-      ax.on = slab_coef<T, false>(d, 0, i, nx - 1, ax.b, ax.c, ax.ik);
-      // Every operand first (all in the padded volumes), then the updates.
-      const T ex0 = ex[c];
-      const T eyk = ey[c + 1], ezj = ez[c + dj], ezi = ez[c + di];
-      const T exk = ex[c + 1], exj = ex[c + dj], eyi = ey[c + di];
-      const T hx0 = hx[c], hy0 = hy[c], hz0 = hz[c];
-      const bool vy = i < nx - 1 && kin, vz = i < nx - 1 && jin;
-      T p_xz = T(0), p_xy = T(0), p_yx = T(0), p_yz = T(0), p_zy = T(0), p_zx = T(0);
-      if (vx && az.on) p_xz = pxz[c];
-      if (vx && ay.on) p_xy = pxy[c];
-      if (vy && ax.on) p_yx = pyx[c];
-      if (vy && az.on) p_yz = pyz[c];
-      if (vz && ay.on) p_zy = pzy[c];
-      if (vz && ax.on) p_zx = pzx[c];
-      if (vx) {  // Hx (nx, ny-1, nz-1): +dt/mu (t_hxz - t_hxy)
-        const T dey_dz = (eyk - ey0) * idz, dez_dy = (ezj - ez0) * idy;
-        T tz = dey_dz, ty = dez_dy;
-        if (az.on) {
-          tz = psi_term(az, dey_dz, p_xz);
-          pxz[c] = p_xz;
-        }
-        if (ay.on) {
-          ty = psi_term(ay, dez_dy, p_xy);
-          pxy[c] = p_xy;
-        }
-        hx[c] = hx0 + dt_mu * (tz - ty);
-      }
-      if (vy) {  // Hy (nx-1, ny, nz-1): +dt/mu (t_hyx - t_hyz)
-        const T dez_dx = (ezi - ez0) * idx, dex_dz = (exk - ex0) * idz;
-        T tx = dez_dx, tz = dex_dz;
-        if (ax.on) {
-          tx = psi_term(ax, dez_dx, p_yx);
-          pyx[c] = p_yx;
-        }
-        if (az.on) {
-          tz = psi_term(az, dex_dz, p_yz);
-          pyz[c] = p_yz;
-        }
-        hy[c] = hy0 + dt_mu * (tx - tz);
-      }
-      if (vz) {  // Hz (nx-1, ny-1, nz): +dt/mu (t_hzy - t_hzx)
-        const T dex_dy = (exj - ex0) * idy, dey_dx = (eyi - ey0) * idx;
-        T ty = dex_dy, tx = dey_dx;
-        if (ay.on) {
-          ty = psi_term(ay, dex_dy, p_zy);
-          pzy[c] = p_zy;
-        }
-        if (ax.on) {
-          tx = psi_term(ax, dey_dx, p_zx);
-          pzx[c] = p_zx;
-        }
-        hz[c] = hz0 + dt_mu * (ty - tx);
-      }
-      ey0 = eyi;
-      ez0 = ezi;
+    const Vec<T> ex0 = ldv(ex + c), exj = ldv(ex + c + dj);
+    const Vec<T> eyi = ldv(ey + c + di), ezi = ldv(ez + c + di), ezj = ldv(ez + c + dj);
+    const T exk = ex[c + V], eyk = ey[c + V];
+    Vec<T> h0 = ldv(hx + c), h1 = ldv(hy + c), h2 = ldv(hz + c);
+    const bool iin = i < nx - 1;
+    const unsigned vx = jin ? kin : 0u, vy = iin ? kin : 0u, vz = iin && jin ? kall : 0u;
+    // psi and the plane's x coefficients with the fields, before any use.
+    const bool xon = in_slab(d.npml, i, nx - 1);
+    const unsigned o_xz = vx & zon, o_xy = yon ? vx : 0u, o_yx = xon ? vy : 0u, o_yz = vy & zon,
+                   o_zy = yon ? vz : 0u, o_zx = xon ? vz : 0u;
+    T* const psi = d.psi + c;
+    Vec<T> p_xz{}, p_xy{}, p_yx{}, p_yz{}, p_zy{}, p_zx{};
+    if (o_xz) p_xz = ldv(psi + P_HXZ * d.vol);
+    if (o_xy) p_xy = ldv(psi + P_HXY * d.vol);
+    if (o_yx) p_yx = ldv(psi + P_HYX * d.vol);
+    if (o_yz) p_yz = ldv(psi + P_HYZ * d.vol);
+    if (o_zy) p_zy = ldv(psi + P_HZY * d.vol);
+    if (o_zx) p_zx = ldv(psi + P_HZX * d.vol);
+    Ax<T> ax{};
+    if (xon) ax = coef_at<T, false>(d, 0, i);
+    Vec<T> d0, d1, d2, d3, d4, d5;  // differences
+#pragma unroll
+    for (int x = 0; x < V; ++x) {
+      d0[x] = sub_(x + 1 < V ? ey0[x + 1 < V ? x + 1 : 0] : eyk, ey0[x]);
+      d1[x] = sub_(ezj[x], ez0[x]);
+      d2[x] = sub_(ezi[x], ez0[x]);
+      d3[x] = sub_(x + 1 < V ? ex0[x + 1 < V ? x + 1 : 0] : exk, ex0[x]);
+      d4[x] = sub_(exj[x], ex0[x]);
+      d5[x] = sub_(eyi[x], ey0[x]);
     }
-    if (fl & F_HPTS) {
-      __syncthreads();
-      T* hs[3] = {hx, hy, hz};
-      for (int t = 3; t < 6; ++t) {
-        const int np_ = t == 3 ? d.n_mx : (t == 4 ? d.n_my : d.n_mz);
-        for (int q = d.off[t][cta] + tid; q < d.off[t][cta + 1]; q += NT) {
-          const Pt3 p = d.pts[t][q];
-          atomicAdd(hs[t - 3] + at(d, p.i, p.j, p.k), -(dt_mu * wave(d, t, np_, p.m, n, sub)));
-        }
+    const unsigned gen = near_slab(d.npml, i, i + 1, nx) ? ALL : th.gen;
+    if ((gen | (ALL ^ kin)) == 0 && iin && jin) {
+      // No slab within reach and every cell live: the bare update.
+#pragma unroll
+      for (int x = 0; x < V; ++x) {
+        h0[x] = fma_(dt_mu, x_bare(d0[x], idz, d1[x], idy), h0[x]);
+        h1[x] = fma_(dt_mu, x_bare(d2[x], idx, d3[x], idz), h1[x]);
+        h2[x] = fma_(dt_mu, x_bare(d4[x], idy, d5[x], idx), h2[x]);
       }
+    } else {
+      const unsigned bare = ~gen;
+      auto part = [&](Vec<T>& h, unsigned valid, const Vec<T>& da, T ia, const Vec<T>& db,
+                      T ib, auto&& terms) {
+        Vec<T> ta, tb;
+#pragma unroll
+        for (int x = 0; x < V; ++x) {
+          ta[x] = mul_(da[x], ia);
+          tb[x] = mul_(db[x], ib);
+        }
+        terms(ta, tb);
+#pragma unroll
+        for (int x = 0; x < V; ++x) {
+          const T X = bare >> x & 1 ? x_bare(da[x], ia, db[x], ib) : sub_(ta[x], tb[x]);
+          if (valid >> x & 1) h[x] = fma_(dt_mu, X, h[x]);
+        }
+      };
+      part(h0, vx, d0, idz, d1, idy, [&](Vec<T>& a, Vec<T>& b) {
+        stretch(az, o_xz, p_xz, a);
+        stretch(ay, o_xy, p_xy, b);
+      });
+      part(h1, vy, d2, idx, d3, idz, [&](Vec<T>& a, Vec<T>& b) {
+        stretch(ax, o_yx, p_yx, a);
+        stretch(az, o_yz, p_yz, b);
+      });
+      part(h2, vz, d4, idy, d5, idx, [&](Vec<T>& a, Vec<T>& b) {
+        stretch(ay, o_zy, p_zy, a);
+        stretch(ax, o_zx, p_zx, b);
+      });
     }
+    if (o_xz) stv(psi + P_HXZ * d.vol, p_xz);
+    if (o_xy) stv(psi + P_HXY * d.vol, p_xy);
+    if (o_yx) stv(psi + P_HYX * d.vol, p_yx);
+    if (o_yz) stv(psi + P_HYZ * d.vol, p_yz);
+    if (o_zy) stv(psi + P_HZY * d.vol, p_zy);
+    if (o_zx) stv(psi + P_HZX * d.vol, p_zx);
+    stv(hx + c, h0);
+    stv(hy + c, h1);
+    stv(hz + c, h2);
+    ey0 = eyi;
+    ez0 = ezi;
   }
 }
 
 // ---------------------------------------------------------------------------
-// E update: H^{n+1/2} -> E^{n+1} (fdtd3d.py:596-633) + sources, port,
-// probes, V/I and E monitors. Same CTA geometry as yee_h.
+// E update: H^{n+1/2} -> E^{n+1} (fdtd3d.py:596-633) + the sources near probes
+// and the port, the port, probes and V/I. Same CTA geometry as yee_h.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3) yee_e(Dev3<T> d, int sub, int ni) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_e(Dev3<T> d, int sub, int ni) {
+  constexpr int V = Vec<T>::V;
+  constexpr unsigned ALL = (1u << V) - 1;
   __shared__ T s_port[3];  // Ez^n, curl_z and the plain-updated Ez at the port edge
   dependent_launch_gate();
   const int n = *d.step_base + sub;
-  const int k = blockIdx.x * BK + threadIdx.x;
-  const int j = blockIdx.y * BJ + threadIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  const bool live = j < ny && k < nz;
-  const int tid = threadIdx.y * BK + threadIdx.x;
-  const int i0 = int(blockIdx.z) * ni, i1 = min(nx, i0 + ni);
+  const int tid = threadIdx.x;
+  const int i0 = int(blockIdx.y) * ni, i1 = min(nx, i0 + ni);
+  const Thread3<T> th = locate(d, i0);
   const int di = d.sy * d.sz, dj = d.sz;
-  int c = ((i0 + 1) * d.sy + (j + 1)) * d.sz + (k + 1);
-  long long g = ((long long)i0 * ny + j) * nz + k;  // node coefficients
-  const long long dgi = (long long)ny * nz;
+  int c = th.c;
   T *ex = d.f[0], *ey = d.f[1], *ez = d.f[2];
   const T* __restrict__ hx = d.f[3];
   const T* __restrict__ hy = d.f[4];
   const T* __restrict__ hz = d.f[5];
-  T *pxy = d.psi + P_EXY * d.vol, *pxz = d.psi + P_EXZ * d.vol, *pyz = d.psi + P_EYZ * d.vol,
-    *pyx = d.psi + P_EYX * d.vol, *pzx = d.psi + P_EZX * d.vol, *pzy = d.psi + P_EZY * d.vol;
   const T idx = d.inv_d[0], idy = d.inv_d[1], idz = d.inv_d[2];
   // E-type samples of this thread's y and z (the PEC interior, node - 1).
-  Ax<T> ay, az;
-  ay.on = slab_coef<T, true>(d, 1, j - 1, ny - 2, ay.b, ay.c, ay.ik);
-  az.on = slab_coef<T, true>(d, 2, k - 1, nz - 2, az.b, az.c, az.ik);
-  const bool jx = j >= 1 && j <= ny - 2, kx = k >= 1 && k <= nz - 2;
-  const bool vx_jk = jx && kx, vy_jk = j < ny - 1 && kx, vz_jk = jx && k < nz - 1;
+  const Ax<T> ay = coef_at<T, true>(d, 1, th.live ? th.j : 0);
+  const Az<T> az = coef_z<T, true>(d, th.k0);
+  const bool yon = in_slab(d.npml, th.j - 1, ny - 2);
+  const unsigned zon = slab_mask<V>(d.npml, th.k0 - 1, nz - 2);
+  const bool jx = th.j >= 1 && th.j <= ny - 2;
+  const unsigned kx = range_mask<V>(th.k0, 1, nz - 1), kin = range_mask<V>(th.k0, 0, nz - 1);
   // Hy and Hz of plane i - 1 (the previous plane's own values).
-  T hyi = T(0), hzi = T(0);
-  if (live) {
-    hyi = hy[c - di];
-    hzi = hz[c - di];
+  Vec<T> hyi{}, hzi{};
+  if (th.live) {
+    hyi = ldv(hy + c - di);
+    hzi = ldv(hz + c - di);
   }
-  for (int i = i0; i < i1; ++i, c += di, g += dgi) {
-    const int cta = (i * d.gj + blockIdx.y) * d.gk + blockIdx.x;
-    const unsigned fl = d.cls[cta];
+  for (int i = i0; i < i1; ++i, c += di) {
+    const int cta = i * int(gridDim.x) + int(blockIdx.x);
     const bool port_here = d.has_port && cta == d.port_cta;
-    if (live && !(fl & F_CPML)) {
-      // No slab within reach of this plane box: the bare update.
-      const T hx0 = hx[c], hy0 = hy[c], hz0 = hz[c];
-      const T hzj = hz[c - dj], hyk = hy[c - 1], hxk = hx[c - 1], hxj = hx[c - dj];
-      const T ex0 = ex[c], ey0 = ey[c], ez0 = ez[c];
-      const T ca = d.ca[g], cb = d.cb[g];
+    if (th.live) {
+      const Vec<T> hx0 = ldv(hx + c), hy0 = ldv(hy + c), hz0 = ldv(hz + c);
+      const Vec<T> hzj = ldv(hz + c - dj), hxj = ldv(hx + c - dj);
+      const T hyk = hy[c - 1], hxk = hx[c - 1];
+      Vec<T> e0 = ldv(ex + c), e1 = ldv(ey + c), e2 = ldv(ez + c);
+      Vec<T> ca, cb;
+      if (d.cap) {
+        ca = ldv(d.cap + c);
+        cb = ldv(d.cbp + c);
+      } else {
+        const long long g = ((long long)i * ny + th.j) * nz + th.k0;
+#pragma unroll
+        for (int x = 0; x < V; ++x) {
+          const bool in = th.k0 + x >= 0 && th.k0 + x < nz;
+          ca[x] = in ? d.ca[g + x] : T(0);
+          cb[x] = in ? d.cb[g + x] : T(0);
+        }
+      }
       const bool iin = i >= 1 && i <= nx - 2;
-      const bool vx = i < nx - 1 && vx_jk, vy = iin && vy_jk, vz = iin && vz_jk;
-      if (vx) ex[c] = ca * ex0 + cb * ((hz0 - hzj) * idy - (hy0 - hyk) * idz);
-      if (vy) ey[c] = ca * ey0 + cb * ((hx0 - hxk) * idz - (hz0 - hzi) * idx);
-      if (vz) {
-        const T curl = (hy0 - hyi) * idx - (hx0 - hxj) * idy;
-        const T upd = ca * ez0 + cb * curl;
-        if (port_here && i == d.pi && j == d.pj && k == d.pk) {
-          s_port[0] = ez0;
-          s_port[1] = curl;
-          s_port[2] = upd;
-        }
-        ez[c] = upd;
+      const unsigned vx = i < nx - 1 && jx ? kx : 0u, vy = iin && th.j < ny - 1 ? kx : 0u,
+                     vz = iin && jx ? kin : 0u;
+      // psi and the plane's x coefficients with the fields, before any use.
+      const bool xon = in_slab(d.npml, i - 1, nx - 2);
+      const unsigned o_xy = yon ? vx : 0u, o_xz = vx & zon, o_yz = vy & zon, o_yx = xon ? vy : 0u,
+                     o_zx = xon ? vz : 0u, o_zy = yon ? vz : 0u;
+      T* const psi = d.psi + c;
+      Vec<T> p_xy{}, p_xz{}, p_yz{}, p_yx{}, p_zx{}, p_zy{};
+      if (o_xy) p_xy = ldv(psi + P_EXY * d.vol);
+      if (o_xz) p_xz = ldv(psi + P_EXZ * d.vol);
+      if (o_yz) p_yz = ldv(psi + P_EYZ * d.vol);
+      if (o_yx) p_yx = ldv(psi + P_EYX * d.vol);
+      if (o_zx) p_zx = ldv(psi + P_EZX * d.vol);
+      if (o_zy) p_zy = ldv(psi + P_EZY * d.vol);
+      Ax<T> ax{};
+      if (xon) ax = coef_at<T, true>(d, 0, i);
+      Vec<T> d0, d1, d2, d3, d4, d5;  // differences
+#pragma unroll
+      for (int x = 0; x < V; ++x) {
+        d0[x] = sub_(hz0[x], hzj[x]);
+        d1[x] = sub_(hy0[x], x > 0 ? hy0[x > 0 ? x - 1 : 0] : hyk);
+        d2[x] = sub_(hx0[x], x > 0 ? hx0[x > 0 ? x - 1 : 0] : hxk);
+        d3[x] = sub_(hz0[x], hzi[x]);
+        d4[x] = sub_(hy0[x], hyi[x]);
+        d5[x] = sub_(hx0[x], hxj[x]);
       }
-      hyi = hy0;
-      hzi = hz0;
-    } else if (live) {
-      Ax<T> ax;
-      ax.on = slab_coef<T, true>(d, 0, i - 1, nx - 2, ax.b, ax.c, ax.ik);
-      const T hx0 = hx[c], hy0 = hy[c], hz0 = hz[c];
-      const T hzj = hz[c - dj], hyk = hy[c - 1], hxk = hx[c - 1], hxj = hx[c - dj];
-      const T ex0 = ex[c], ey0 = ey[c], ez0 = ez[c];
-      const T ca = d.ca[g], cb = d.cb[g];
-      const bool iin = i >= 1 && i <= nx - 2;
-      const bool vx = i < nx - 1 && vx_jk, vy = iin && vy_jk, vz = iin && vz_jk;
-      T p_xy = T(0), p_xz = T(0), p_yz = T(0), p_yx = T(0), p_zx = T(0), p_zy = T(0);
-      if (vx && ay.on) p_xy = pxy[c];
-      if (vx && az.on) p_xz = pxz[c];
-      if (vy && az.on) p_yz = pyz[c];
-      if (vy && ax.on) p_yx = pyx[c];
-      if (vz && ax.on) p_zx = pzx[c];
-      if (vz && ay.on) p_zy = pzy[c];
-      if (vx) {  // Ex (nx-1, ny, nz) interior j, k: t_exy - t_exz
-        const T dhz_dy = (hz0 - hzj) * idy, dhy_dz = (hy0 - hyk) * idz;
-        T ty = dhz_dy, tz = dhy_dz;
-        if (ay.on) {
-          ty = psi_term(ay, dhz_dy, p_xy);
-          pxy[c] = p_xy;
+      Vec<T> old, curl;
+      if (port_here) old = e2;
+      const unsigned gen = near_slab(d.npml, i, i + 1, nx) ? ALL : th.gen;
+      if ((gen | (ALL ^ kx)) == 0 && iin && jx) {
+        // No slab within reach and every cell live: the bare update.
+#pragma unroll
+        for (int x = 0; x < V; ++x) {
+          e0[x] = e_next(ca[x], e0[x], cb[x], x_bare(d0[x], idy, d1[x], idz));
+          e1[x] = e_next(ca[x], e1[x], cb[x], x_bare(d2[x], idz, d3[x], idx));
+          curl[x] = x_bare(d4[x], idx, d5[x], idy);
+          e2[x] = e_next(ca[x], e2[x], cb[x], curl[x]);
         }
-        if (az.on) {
-          tz = psi_term(az, dhy_dz, p_xz);
-          pxz[c] = p_xz;
-        }
-        ex[c] = ca * ex0 + cb * (ty - tz);
+      } else {
+        const unsigned bare = ~gen;
+        auto part = [&](Vec<T>& e, unsigned valid, const Vec<T>& da, T ia,
+                        const Vec<T>& db, T ib, auto&& terms) {
+          Vec<T> ta, tb;
+#pragma unroll
+          for (int x = 0; x < V; ++x) {
+            ta[x] = mul_(da[x], ia);
+            tb[x] = mul_(db[x], ib);
+          }
+          terms(ta, tb);
+#pragma unroll
+          for (int x = 0; x < V; ++x) {
+            ta[x] = bare >> x & 1 ? x_bare(da[x], ia, db[x], ib) : sub_(ta[x], tb[x]);
+            if (valid >> x & 1) e[x] = e_next(ca[x], e[x], cb[x], ta[x]);
+          }
+          return ta;
+        };
+        part(e0, vx, d0, idy, d1, idz, [&](Vec<T>& a, Vec<T>& b) {
+          stretch(ay, o_xy, p_xy, a);
+          stretch(az, o_xz, p_xz, b);
+        });
+        part(e1, vy, d2, idz, d3, idx, [&](Vec<T>& a, Vec<T>& b) {
+          stretch(az, o_yz, p_yz, a);
+          stretch(ax, o_yx, p_yx, b);
+        });
+        curl = part(e2, vz, d4, idx, d5, idy, [&](Vec<T>& a, Vec<T>& b) {
+          stretch(ax, o_zx, p_zx, a);
+          stretch(ay, o_zy, p_zy, b);
+        });
       }
-      if (vy) {  // Ey (nx, ny-1, nz) interior i, k: t_eyz - t_eyx
-        const T dhx_dz = (hx0 - hxk) * idz, dhz_dx = (hz0 - hzi) * idx;
-        T tz = dhx_dz, tx = dhz_dx;
-        if (az.on) {
-          tz = psi_term(az, dhx_dz, p_yz);
-          pyz[c] = p_yz;
-        }
-        if (ax.on) {
-          tx = psi_term(ax, dhz_dx, p_yx);
-          pyx[c] = p_yx;
-        }
-        ey[c] = ca * ey0 + cb * (tz - tx);
+      if (port_here && i == d.pi && th.j == d.pj) {
+#pragma unroll
+        for (int x = 0; x < V; ++x)
+          if (th.k0 + x == d.pk) {
+            s_port[0] = old[x];
+            s_port[1] = curl[x];
+            s_port[2] = e2[x];
+          }
       }
-      if (vz) {  // Ez (nx, ny, nz-1) interior i, j: t_ezx - t_ezy
-        const T dhy_dx = (hy0 - hyi) * idx, dhx_dy = (hx0 - hxj) * idy;
-        T tx = dhy_dx, ty = dhx_dy;
-        if (ax.on) {
-          tx = psi_term(ax, dhy_dx, p_zx);
-          pzx[c] = p_zx;
-        }
-        if (ay.on) {
-          ty = psi_term(ay, dhx_dy, p_zy);
-          pzy[c] = p_zy;
-        }
-        const T curl = tx - ty;
-        const T upd = ca * ez0 + cb * curl;
-        if (port_here && i == d.pi && j == d.pj && k == d.pk) {
-          s_port[0] = ez0;
-          s_port[1] = curl;
-          s_port[2] = upd;
-        }
-        ez[c] = upd;
-      }
+      if (o_xy) stv(psi + P_EXY * d.vol, p_xy);
+      if (o_xz) stv(psi + P_EXZ * d.vol, p_xz);
+      if (o_yz) stv(psi + P_EYZ * d.vol, p_yz);
+      if (o_yx) stv(psi + P_EYX * d.vol, p_yx);
+      if (o_zx) stv(psi + P_EZX * d.vol, p_zx);
+      if (o_zy) stv(psi + P_EZY * d.vol, p_zy);
+      stv(ex + c, e0);
+      stv(ey + c, e1);
+      stv(ez + c, e2);
       hyi = hy0;
       hzi = hz0;
     }
-    if (fl & F_EPTS) {
+    if (d.cls[cta] & F_EPTS) {
       __syncthreads();
       T* es[3] = {ez, ex, ey};  // point types 0 src (Jz), 1 jx, 2 jy
       const T* cbs[3] = {d.cb_src, d.cb_jx, d.cb_jy};
@@ -550,6 +733,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3) yee_e(Dev3<T> d, i
     }
   }
 }
+
 
 // DFT fold over `cnt` ring slots (fdtd3d.py:635-662).
 template <typename T, typename A, int KM>
@@ -724,9 +908,11 @@ static void comp_shape(int c, int nx, int ny, int nz, int s[3]) {
 }
 
 struct Layout3 {
-  int sy = 0, sz = 0, gj = 0, gk = 0, n_cta = 0, R = 32;
+  int sy = 0, sz = 0, tw = 0, cols = 0, n_cta = 0, R = 32;
+  bool coef = false;  // padded copies of ca, cb
+  int ts = 0;         // length of a CPML table
   long long vol = 0, mon_cells = 0;
-  size_t fields, psi, zero_end, off[7], pts[7], pcomp, fpts, mons, gsrc, mring, step, eacc, cwv,
+  size_t fields, psi, cap, tab, zero_end, off[7], pts[7], pcomp, fpts, mons, gsrc, mring, step, eacc, cwv,
       cls, total;
 };
 
@@ -779,14 +965,17 @@ static int count_of(const GdnYeeParams* p, int t) {
   return a[t];
 }
 
-static Layout3 make_layout3(const GdnYeeParams* p, const GdnYeePoints* pts, size_t esize) {
+static Layout3 make_layout3(const GdnYeeParams* p, const GdnYeePoints* pts, size_t esize,
+                            bool coef = true) {
   Layout3 L;
   L.sz = int(div_up(p->nz + 2, 4) * 4);
   L.sy = p->ny + 2;
   L.vol = (long long)(p->nx + 2) * L.sy * L.sz;
-  L.gk = int(div_up(p->nz, BK));
-  L.gj = int(div_up(p->ny, BJ));
-  L.n_cta = p->nx * L.gj * L.gk;
+  L.tw = int(div_up(p->nz + 1, 16 / (long long)esize));
+  L.cols = int(div_up((long long)p->ny * L.tw, NT));
+  L.n_cta = p->nx * L.cols;
+  // Runs whose volumes take most of the card read the caller's ca, cb instead.
+  L.coef = coef && 20 * L.vol * (long long)esize <= (48LL << 30);
   L.mon_cells = pts ? mon_cells3(p, pts) : 0;
   const size_t budget = size_t(2) << 30;
   long long r = L.mon_cells > 0 ? (long long)(budget / (size_t(L.mon_cells) * esize)) : 32;
@@ -795,6 +984,9 @@ static Layout3 make_layout3(const GdnYeeParams* p, const GdnYeePoints* pts, size
   L.fields = cv.take<char>(size_t(NC) * L.vol * esize);
   L.psi = cv.take<char>(size_t(12) * L.vol * esize);
   L.step = cv.take<int>(1);
+  L.cap = cv.take<char>(L.coef ? 2 * size_t(L.vol) * esize : 0);
+  L.ts = int(div_up(std::max({p->nx, p->ny, p->nz}) + 8, 4) * 4);
+  L.tab = cv.take<char>(18 * size_t(L.ts) * esize);
   L.zero_end = cv.take<char>(0);
   for (int t = 0; t < 7; ++t) {
     L.off[t] = cv.take<int>(L.n_cta + 1);
@@ -917,8 +1109,11 @@ static void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStre
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Planes per CTA for a step kernel: the CTAs of `cols` (j, k) tile columns
-// split the nx planes so that the whole grid is one wave of resident CTAs.
+// Planes per CTA for a step kernel: as few as let every CTA of the `cols`
+// column blocks be resident at once, two at most. Each plane is a trip to L2
+// that only other warps hide: at 160 x 160 x 64 f32 a step with 7 planes a CTA
+// (one wave) takes 53 us, with two (three waves) 50, with one 54; at 97 x 83 x
+// 61 four planes instead of two cost a quarter more.
 template <typename K>
 static int planes_per_cta(K kernel, int nx, int cols, int* ni) {
   int dev = 0, sms = 0, per_sm = 0;
@@ -927,7 +1122,7 @@ static int planes_per_cta(K kernel, int nx, int cols, int* ni) {
   GDN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, 0));
   const long long slots = (long long)std::max(sms, 1) * std::max(per_sm, 1);
   const long long per_col = std::max<long long>(1, slots / std::max(cols, 1));
-  *ni = int(std::max<long long>(1, div_up(nx, per_col)));
+  *ni = int(std::min<long long>(2, std::max<long long>(1, div_up(nx, per_col))));
   return GDN_OK;
 }
 
@@ -951,14 +1146,25 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
                 cudaStream_t stream) {
   int st = validate3(p, pts, b);
   if (st) return st;
-  const Layout3 L = make_layout3(p, pts, sizeof(T));
+  Layout3 L = make_layout3(p, pts, sizeof(T));
   char* ws = static_cast<char*>(b->workspace);
   bool own = false;
-  if (!ws) {
-    GDN_TRY_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&ws), L.total, stream));
+  if (ws && b->workspace_bytes < L.total) {
+    // Scratch that does without the padded ca, cb is enough.
+    L = make_layout3(p, pts, sizeof(T), false);
+    if (b->workspace_bytes < L.total)
+      GDN_BAD_ARG("workspace too small: %zu < %zu bytes", b->workspace_bytes, L.total);
+  }
+  // Vectors need 16-byte boundaries; a caller's scratch may lie elsewhere.
+  if (!ws || reinterpret_cast<uintptr_t>(ws) % 16) {
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ws), L.total, stream);
+    if (e == cudaErrorMemoryAllocation && L.coef) {
+      cudaGetLastError();
+      L = make_layout3(p, pts, sizeof(T), false);
+      e = cudaMallocAsync(reinterpret_cast<void**>(&ws), L.total, stream);
+    }
+    GDN_TRY_CUDA(e);
     own = true;
-  } else if (b->workspace_bytes < L.total) {
-    GDN_BAD_ARG("workspace too small: %zu < %zu bytes", b->workspace_bytes, L.total);
   }
   struct Guard {
     char* p;
@@ -972,7 +1178,7 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
   const int nx = p->nx, ny = p->ny, nz = p->nz, N = p->n_steps;
   Dev3<T> d{};
   d.nx = nx; d.ny = ny; d.nz = nz; d.npml = p->npml; d.n_steps = N; d.n_freq = p->n_freq;
-  d.R = L.R; d.gj = L.gj; d.gk = L.gk; d.sy = L.sy; d.sz = L.sz; d.vol = L.vol;
+  d.R = L.R; d.tw = L.tw; d.sy = L.sy; d.sz = L.sz; d.vol = L.vol;
   for (int c = 0; c < NC; ++c) d.f[c] = reinterpret_cast<T*>(ws + L.fields) + c * L.vol;
   d.psi = reinterpret_cast<T*>(ws + L.psi);
   d.ca = static_cast<const T*>(b->ca);
@@ -1000,7 +1206,12 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
   d.n_mx = p->n_mx; d.n_my = p->n_my; d.n_mz = p->n_mz; d.n_probes = p->n_probes;
   d.has_port = p->has_port;
   d.pi = pts->port[0]; d.pj = pts->port[1]; d.pk = pts->port[2];
-  d.port_cta = p->has_port ? (d.pi * L.gj + d.pj / BJ) * L.gk + d.pk / BK : -1;
+  // CTA that owns a cell: NT vectors of V cells of a plane's rows.
+  constexpr int V = 16 / int(sizeof(T));
+  auto box_of = [&](int i, int j, int k) {
+    return i * L.cols + int(((long long)j * L.tw + (k + 1) / V) / NT);
+  };
+  d.port_cta = p->has_port ? box_of(d.pi, d.pj, d.pk) : -1;
   d.cb_src = static_cast<const T*>(b->cb_src);
   d.cb_jx = static_cast<const T*>(b->cb_jx);
   d.cb_jy = static_cast<const T*>(b->cb_jy);
@@ -1035,10 +1246,9 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
     if (p->cw_sources) d.cw_total += count_of(p, t);
   }
 
-  // Point bins by CTA box (i, j/BJ, k/BK). E sources stay in the step
-  // kernel only in boxes that hold probes or the port; every other source
-  // point goes to the injection lists.
-  auto box_of = [&](int i, int j, int k) { return (i * L.gj + j / BJ) * L.gk + k / BK; };
+  // Point bins by CTA and plane. E sources stay in the step kernel only where
+  // their CTA also has probes or the port; every other source point goes to the
+  // injection lists.
   std::vector<unsigned char> keep_box(L.n_cta, 0);
   for (int m = 0; m < p->n_probes; ++m)
     keep_box[box_of(pts->probe[3 * m], pts->probe[3 * m + 1], pts->probe[3 * m + 2])] = 1;
@@ -1145,9 +1355,7 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
   }
   d.n_mons = int(mons.size());
   d.mons = reinterpret_cast<const Mon3*>(ws + L.mons);
-  // Work flags per plane box: points of the H or E kernel (the port's box
-  // counts as E points) and any CPML slab within reach of the box (either
-  // field type, a margin of one cell).
+  // Points and the port, by the CTA and plane that apply them.
   {
     std::vector<unsigned char> cls(L.n_cta, 0);
     for (int t = 0; t < 7; ++t) {
@@ -1155,22 +1363,10 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
       const int32_t* a = pts_of(pts, t);
       for (int m = 0; m < n; ++m) {
         const int c = box_of(a[3 * m], a[3 * m + 1], a[3 * m + 2]);
-        if (in_kernel(t, c)) cls[c] |= (t >= 3 && t <= 5) ? F_HPTS : F_EPTS;
+        if (in_kernel(t, c)) cls[c] = F_EPTS;
       }
     }
-    if (p->has_port) cls[d.port_cta] |= F_EPTS;
-    const int m = p->npml;
-    auto near_slab = [m](int lo, int hi, int n) {  // cells [lo, hi) of an axis of n nodes
-      return lo <= m + 1 || hi - 1 >= n - 2 - m;
-    };
-    for (int i = 0; i < nx; ++i)
-      for (int by = 0; by < L.gj; ++by)
-        for (int bx = 0; bx < L.gk; ++bx) {
-          const bool sl = m > 0 && (near_slab(i, i + 1, nx) ||
-                                    near_slab(by * BJ, std::min(ny, (by + 1) * BJ), ny) ||
-                                    near_slab(bx * BK, std::min(nz, (bx + 1) * BK), nz));
-          if (sl) cls[(i * L.gj + by) * L.gk + bx] |= F_CPML;
-        }
+    if (p->has_port) cls[d.port_cta] = F_EPTS;
     GDN_TRY_CUDA(cudaMemcpyAsync(ws + L.cls, cls.data(), cls.size(), cudaMemcpyHostToDevice,
                                  stream));
     d.cls = reinterpret_cast<const unsigned char*>(ws + L.cls);
@@ -1197,14 +1393,30 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
   if (p->record_energy)
     GDN_TRY_CUDA(cudaMemsetAsync(eacc, 0, 2 * size_t(std::max(N, 1)) * sizeof(double), stream));
 
-  const dim3 blk(BK, BJ);
+  d.ts = L.ts;
+  d.tab = reinterpret_cast<T*>(ws + L.tab);
+  yee_tables<T><<<dim3(unsigned(div_up(L.ts, 128)), 3), 128, 0, stream>>>(
+      d, reinterpret_cast<T*>(ws + L.tab));
+  count_launches(1);
+  if (L.coef) {
+    T* const cap = reinterpret_cast<T*>(ws + L.cap);
+    if (b->state_in)
+      GDN_TRY_CUDA(cudaMemsetAsync(cap, 0, 2 * size_t(L.vol) * sizeof(T), stream));
+    d.cap = cap;
+    d.cbp = cap + L.vol;
+    yee_pad_coef<T><<<int(std::min<long long>(div_up((long long)nx * ny * nz, 256), 148 * 8)), 256, 0,
+                      stream>>>(d, cap, cap + L.vol);
+    count_launches(1);
+  }
+
+  const dim3 blk(NT);
   // Planes per CTA: the fewest that fit every CTA of the grid into one wave
   // of resident CTAs (a partial second wave would idle most SMs).
   int ni_h = 0, ni_e = 0;
-  if ((st = planes_per_cta(yee_h<T>, nx, L.gj * L.gk, &ni_h))) return st;
-  if ((st = planes_per_cta(yee_e<T>, nx, L.gj * L.gk, &ni_e))) return st;
-  const dim3 grd_h(L.gk, L.gj, unsigned(div_up(nx, ni_h)));
-  const dim3 grd_e(L.gk, L.gj, unsigned(div_up(nx, ni_e)));
+  if ((st = planes_per_cta(yee_h<T>, nx, L.cols, &ni_h))) return st;
+  if ((st = planes_per_cta(yee_e<T>, nx, L.cols, &ni_e))) return st;
+  const dim3 grd_h(unsigned(L.cols), unsigned(div_up(nx, ni_h)));
+  const dim3 grd_e(unsigned(L.cols), unsigned(div_up(nx, ni_e)));
   const int eblocks = int(std::min<long long>(div_up((long long)nx * ny * nz, 256), 148 * 8));
   // Chunk body. With a side stream the ring gathers run beside the step
   // kernels: a gather only reads the field it copies, so the H gather of
@@ -1237,7 +1449,7 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
     const unsigned gb0 = unsigned(div_up(d.gcells[0], 256)), gb1 = unsigned(div_up(d.gcells[1], 256));
     for (int t = 0; t < cnt; ++t) {
       settle(pend_h, 1);
-      launch_pdl(yee_h<T>, grd_h, blk, s, d, t, ni_h);
+      launch_pdl(yee_h<T>, grd_h, blk, s, d, ni_h);
       k += 1;
       if (d.n_fp[1] > 0) {
         launch_pdl(yee_inject<T>, dim3(unsigned(div_up(d.n_fp[1], 256))), dim3(256), s, d, t, 1);
