@@ -20,12 +20,13 @@
 //   What bounds it: the L2 round trip of a plane's loads with 16 warps an SM
 // (ncu at 160 x 160 x 64 f32: issue 12 %, long-scoreboard stalls 70 %, H 18 us
 // and E 21 us a step; their 160 MB at L2 rates would take about 20 us a step).
+// Coefficients are fetched before the wait for the previous kernel (300 -> 288 ms).
 // One cell a thread, 8 x 32 boxes, was issue bound: 252 (H) and 300 (E) warp
 // instructions per 32 cells. More warps with fewer registers lose to spills (5
 // CTAs an SM: 390 ms for the run of 3 below, 6: 435), 8-byte vectors with 6: 317.
-//   Measured, whole calls:  97 x 83 x 61 f32, 600 steps            13.6 -> 10.6 ms
-//                           64 x 64 x 48 f64, 400 steps             8.5 -> 7.2 ms
-//                           160 x 160 x 64 f32 gradient, 2 x 3000   344 -> 300 ms
+//   Measured, whole calls:  97 x 83 x 61 f32, 600 steps            13.7 -> 10.1 ms
+//                           64 x 64 x 48 f64, 400 steps             8.5 -> 7.0 ms
+//                           160 x 160 x 64 f32 gradient, 2 x 3000   346 -> 288 ms
 //   Point work (sources near probes, the port, probes) is binned by plane and
 // CTA on the host and applied by the owner after its sweep. The running DFT uses
 // the monitor ring of the 2D path: after each half step a gather kernel copies
@@ -448,11 +449,9 @@ template <typename T>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, int ni) {
   constexpr int V = Vec<T>::V;
   constexpr unsigned ALL = (1u << V) - 1;
-  dependent_launch_gate();
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int i0 = int(blockIdx.y) * ni, i1 = min(nx, i0 + ni);
   const Thread3<T> th = locate(d, i0);
-  if (!th.live) return;
   // 32-bit cell offsets (a padded volume holds fewer than 2^31 cells).
   const int di = d.sy * d.sz, dj = d.sz;
   int c = th.c;
@@ -462,12 +461,16 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, i
   T *hx = d.f[3], *hy = d.f[4], *hz = d.f[5];
   const T dt_mu = d.dt_mu, idx = d.inv_d[0], idy = d.inv_d[1], idz = d.inv_d[2];
   // This thread's y and z CPML samples (H-type) are fixed over the planes.
-  const Ax<T> ay = coef_at<T, false>(d, 1, th.j);
+  const Ax<T> ay = coef_at<T, false>(d, 1, th.live ? th.j : 0);
   const Az<T> az = coef_z<T, false>(d, th.k0);
   const bool yon = in_slab(d.npml, th.j, ny - 1);
   const unsigned zon = slab_mask<V>(d.npml, th.k0, nz - 1);
   const bool jin = th.j < ny - 1;
   const unsigned kin = range_mask<V>(th.k0, 0, nz - 1), kall = range_mask<V>(th.k0, 0, nz);
+  // The tables are older than the chunk: only what follows needs the previous
+  // kernel.
+  dependent_launch_gate();
+  if (!th.live) return;
   // Ey and Ez of plane i + 1 become plane i + 1's own values next iteration.
   Vec<T> ey0 = ldv(ey + c), ez0 = ldv(ez + c);
   for (int i = i0; i < i1; ++i, c += di) {
@@ -563,8 +566,6 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_e(Dev3<T> d, i
   constexpr int V = Vec<T>::V;
   constexpr unsigned ALL = (1u << V) - 1;
   __shared__ T s_port[3];  // Ez^n, curl_z and the plain-updated Ez at the port edge
-  dependent_launch_gate();
-  const int n = *d.step_base + sub;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int tid = threadIdx.x;
   const int i0 = int(blockIdx.y) * ni, i1 = min(nx, i0 + ni);
@@ -583,6 +584,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_e(Dev3<T> d, i
   const unsigned zon = slab_mask<V>(d.npml, th.k0 - 1, nz - 2);
   const bool jx = th.j >= 1 && th.j <= ny - 2;
   const unsigned kx = range_mask<V>(th.k0, 1, nz - 1), kin = range_mask<V>(th.k0, 0, nz - 1);
+  dependent_launch_gate();  // the tables are older than the chunk
+  const int n = *d.step_base + sub;
   // Hy and Hz of plane i - 1 (the previous plane's own values).
   Vec<T> hyi{}, hzi{};
   if (th.live) {
