@@ -183,3 +183,11 @@ def tm_loop_stats(reset: bool = True):
     check(load().gdn_tm_loop_stats(ctypes.byref(ms), ctypes.byref(cs), ctypes.byref(nb),
                                    int(reset)))
     return ms.value, cs.value, nb.value
+
+
+def tm_timeouts(reset: bool = True) -> int:
+    """2D runs on the current device that gave up on a wait since the last reset
+    (gdn_tm_status); all outputs of such a run are NaN."""
+    n = c_int32()
+    check(load().gdn_tm_status(ctypes.byref(n), int(reset)))
+    return n.value

@@ -791,6 +791,22 @@ __global__ void tm_copy_out(const T* slot, long long plane, int nx, int ny, int 
   }
 }
 
+// Resident runs that gave up on a wait (gdn_tm_status).
+__device__ int g_gave_up = 0;
+
+// The per-step records of a run that gave up: NaN, like its fields and phasors.
+template <typename T>
+__global__ void tm_void_records(const int* err, T* a, long long na, T* b, long long nb, T* c,
+                                long long nc) {
+  if (!*err) return;
+  const long long g0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  if (g0 == 0) atomicAdd(&g_gave_up, 1);
+  for (long long g = g0; g < na; g += step) a[g] = T(NAN);
+  for (long long g = g0; g < nb; g += step) b[g] = T(NAN);
+  for (long long g = g0; g < nc; g += step) c[g] = T(NAN);
+}
+
 template <typename C>
 __global__ void tm_dft_scale(C* a, long long count, double s, const int* err) {
   if (err && *err) s = NAN;
@@ -1865,6 +1881,12 @@ static int finalize(const GdnTmParams* p, const GdnTmBuffers* b, const Run<T>& R
       tm_dft_scale<float2><<<blocks, 256, 0, stream>>>(static_cast<float2*>(m.out), cnt, p->dt,
                                                       R.err);
   }
+  if (R.err && N > 0) {
+    tm_void_records<T><<<148, 256, 0, stream>>>(
+        R.err, static_cast<T*>(b->out_probe), (long long)N * p->n_probes, static_cast<T*>(b->out_v),
+        (long long)N * p->n_ports, static_cast<T*>(b->out_i), (long long)N * p->n_ports);
+    count_launches(1);
+  }
   if (p->record_energy && N > 0)
     tm_energy_finish<T><<<unsigned(div_up(N, 256)), 256, 0, stream>>>(
         R.eacc, static_cast<T*>(b->out_energy), N, p->dx * p->dy, p->mu0);
@@ -2210,6 +2232,11 @@ static void launch_seg_fold(const Wave<T>& w, int seg0, cudaStream_t s) {
     launch_seg_fold_nc<T, A, KMAX, 1>(w, seg0, s);
 }
 
+// Tests: the block whose words rectangle 0 keeps back in resident runs that this
+// thread starts, or -1 (gdn_tm_inject_timeout).
+static thread_local int t_hold = -1;
+constexpr int kHoldPolls = 1 << 12;  // then a few milliseconds of polls
+
 // All time steps of a wave: per segment the value table, the tiles (one
 // cooperative launch when they all fit, else one launch per block) and the
 // DFT sums.
@@ -2230,7 +2257,7 @@ static int run_wave(const Wave<T>& w, cudaStream_t stream) {
         ++k;
       }
       const int b0 = seg0 / res::TB, b1 = int(div_up(seg0 + cnt, res::TB));
-      res::RArgs<T> a{w.devs, w.tiles, w.err, b0, b1, seg0};
+      res::RArgs<T> a{w.devs, w.tiles, w.err, b0, b1, seg0, t_hold < 0 ? res::POLLS : kHoldPolls, t_hold};
       if ((st = launch_coop<S, S2>(a, w.n_tiles, w.smem, stream))) return st;
       ++k;
       if (w.f64) launch_seg_fold<T, double>(w, seg0, stream);
@@ -2609,6 +2636,22 @@ extern "C" int gdn_tm_run_batch_f32(const GdnTmProblem* problems, int32_t n, int
 extern "C" int gdn_tm_run_f64(const GdnTmParams* p, const GdnTmPoints* pts,
                               const GdnTmBuffers* b, void* stream) {
   return gdn::tm2d::run<double>(p, pts, b, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int gdn_tm_status(int32_t* timeouts, int32_t reset) {
+  using namespace gdn;
+  if (!timeouts) GDN_BAD_ARG("null pointer");
+  GDN_TRY_CUDA(cudaMemcpyFromSymbol(timeouts, tm2d::g_gave_up, sizeof(int32_t)));
+  if (reset) {
+    const int32_t zero = 0;
+    GDN_TRY_CUDA(cudaMemcpyToSymbol(tm2d::g_gave_up, &zero, sizeof(zero)));
+  }
+  return GDN_OK;
+}
+
+extern "C" int gdn_tm_inject_timeout(int32_t block) {
+  gdn::tm2d::t_hold = block < 0 ? -1 : block;
+  return GDN_OK;
 }
 
 // ===========================================================================

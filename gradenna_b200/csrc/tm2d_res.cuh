@@ -45,7 +45,7 @@ namespace res {
 constexpr int TB = 4;
 constexpr int SEG_MAX = 1024;        // steps per segment
 constexpr int FOLD = 32;             // steps per partial DFT sum
-constexpr long long POLLS = 1LL << 22;  // polls of a word before a CTA gives up (seconds)
+constexpr int POLLS = 1 << 22;       // polls of a word before a CTA gives up (seconds)
 
 // A rectangle of owned cells, all of one class.
 struct Rect {
@@ -101,6 +101,8 @@ struct RArgs {
   const RTile* tiles;
   int* err;
   int blk0, blk1, seg0;  // blocks [blk0, blk1); ring and value slot 0 is step seg0
+  int polls;             // polls of a word before a CTA gives up
+  int hold;              // tests: rectangle 0 keeps this block's words back (-1: none)
 };
 
 // NW warps of R rows, V columns a lane.
@@ -612,7 +614,8 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
   };
   // Halo cells from their owners' words of block `blk`, all warps sharing the
   // polls, up to B units in flight; false when a word did not come in time or
-  // another CTA gave up.
+  // another CTA gave up (every rectangle then leaves, and the host makes the
+  // run's outputs NaN).
   auto receive = [&](const uint4* x, unsigned blk) -> bool {
     T* const st = sm + S::O_B;
     const int n = int(d.plane), h = tl.h + 2 * TB, w = tl.w + 2 * TB;
@@ -633,7 +636,7 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
             if (GEN && (U.ie + r < 0 || U.ie + r >= d.nx || U.je + c < 0 || U.je + c >= d.ny)) o[q] |= 1 << 30;
           });
       }
-      long long i = 0;
+      int i = 0;
       unsigned bad;
       do {
         bad = 0;
@@ -672,7 +675,7 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
               }
             }
         }
-        if (bad && (++i >= POLLS || ((i & 255) == 0 && *reinterpret_cast<const volatile int*>(a.err))))
+        if (bad && (++i >= a.polls || ((i & 255) == 0 && *reinterpret_cast<const volatile int*>(a.err))))
           return false;
       } while (bad);
     }
@@ -1050,7 +1053,7 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
     // to the other state slot ----
     if (b + 1 == min(a.blk1, (d.n_steps + TB - 1) / TB))
       store((b & 1) ^ 1);
-    else
+    else if (tl.idx != 0 || b + 1 != a.hold)
       send(D.xch + (long long)((b & 1) ^ 1) * (S::NF + 2 * S::NP) * d.plane, unsigned(b + 1));
     __syncthreads();
   }
@@ -1064,6 +1067,8 @@ __global__ void __launch_bounds__(S::NT, 1) tm_res(RArgs<typename S::T> a) {
   __shared__ __align__(16) unsigned char sdev[sizeof(RDev<T>)];
   __shared__ TileInfo<T> U;
   const RTile tl = a.tiles[blockIdx.x];
+  // A rectangle of an earlier segment (or of this one) gave up: nothing to do.
+  if (__syncthreads_or(*reinterpret_cast<const volatile int*>(a.err))) return;
   const int* src = reinterpret_cast<const int*>(a.devs + tl.prob);
   for (int q = threadIdx.x; q < int(sizeof(RDev<T>) / sizeof(int)); q += S::NT)
     reinterpret_cast<int*>(sdev)[q] = src[q];

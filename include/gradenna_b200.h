@@ -175,6 +175,17 @@ int gdn_tm_run_f32(const GdnTmParams* p, const GdnTmPoints* pts,
 int gdn_tm_run_f64(const GdnTmParams* p, const GdnTmPoints* pts,
                    const GdnTmBuffers* b, void* stream);
 
+/* Number of 2D runs on the current device, since the last reset, that gave up
+ * on a bounded wait between two parts of the grid (0 in normal operation);
+ * synchronises with the device. Every output of such a run is NaN. */
+int gdn_tm_status(int32_t* timeouts, int32_t reset);
+
+/* Test hook for that path: in the 2D runs that the calling thread starts, one
+ * part of the grid keeps back the cells that its neighbours need for the
+ * four-step block `block` (>= 1), and the waits are a few milliseconds long.
+ * -1 (the default) switches the hook off. */
+int gdn_tm_inject_timeout(int32_t block);
+
 /* One problem of a batched run: the same three structs as gdn_tm_run_f32. */
 typedef struct GdnTmProblem {
   const GdnTmParams* params;
