@@ -859,9 +859,11 @@ struct Region {
 struct Plan {
   std::vector<Region> regions;
   int n_rects = 0;
-  size_t smem = 0;  // dynamic shared memory of a CTA
+  size_t smem = 0;  // dynamic shared memory of a CTA without staged values
   bool fits = false;
 };
+constexpr size_t kResSmem = size_t(220) << 10;  // most of it, staged values included
+constexpr size_t kMinStage = 4096;              // staged values at least
 
 static int sm_count() {
   int dev = 0, sms = 0;
@@ -920,7 +922,7 @@ static Plan make_plan(const GdnTmParams* p, size_t esize, const Cfg& c, int kind
     add(r0, c1, r1 - r0, ny - c1, 1);
     add(r0, c0, r1 - r0, c1 - c0, 0);
   }
-  pl.fits = pl.smem <= size_t(220) << 10;
+  pl.fits = pl.smem + kMinStage <= kResSmem;
   return pl;
 }
 
@@ -2011,6 +2013,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   };
   std::vector<std::vector<Copy>> in(nr);
   bool any = false;
+  size_t most = 0;  // injections of a rectangle
   for (int k = 0; k < 5; ++k)
     for (int m = 0; m < counts[k]; ++m) {
       const int i = is[k][m], j = js[k][m], halo = k < 4 ? res::TB : 0;
@@ -2021,13 +2024,15 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
         in[idx].push_back(Copy{k, m, i, j, own});
       });
     }
+  for (const auto& v : in)
+    most = std::max(most, size_t(std::count_if(v.begin(), v.end(), [](const Copy& q) { return q.type < 4; })));
+  const int staged = int(std::min(most, (kResSmem - pl.smem) / (res::TB * sizeof(T))));
   std::vector<res::RHdr> hdr;
   std::vector<int> vl_off(nr + 1, 0), vl, pts_off(1, 0);
   std::vector<res::RPt> ents;
   if (any) {
     const ShapeInfo main = kind_shape(sizeof(T), L.kind, false);
     std::vector<int> cnt(size_t(main.nt) * 4);
-    const int staged = 4096 / int(sizeof(T)) / res::TB;  // values a rectangle stages
     int slots = 0;
     for (int t = 0; t < nr; ++t) {
       if (!in[t].empty()) {
@@ -2128,7 +2133,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
     }
   }
   R.rtiles = std::move(tiles);
-  R.rsmem = pl.smem;
+  R.rsmem = pl.smem + size_t(staged) * res::TB * sizeof(T);
 
   res::RDev<T>& rd = R.rd;
   const size_t a_rd = append(blob, &rd, 1), a_tiles = append(blob, R.rtiles.data(), R.rtiles.size());
@@ -2146,6 +2151,8 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   rd.pv = reinterpret_cast<const T*>(ws + L.pv);
   rd.n_inj = int(injections(p));
   rd.dft_f64 = p->dft_f64 != 0;
+  rd.val_at = int(pl.smem / sizeof(T));
+  rd.val_cap = staged;
   rd.d = d;
   std::copy_n(reinterpret_cast<const char*>(&rd), sizeof(rd), blob.data() + a_rd);
   if (blob.size() > L.blob_bytes)
@@ -2247,7 +2254,7 @@ static int run_wave(const Wave<T>& w, cudaStream_t stream) {
     using S2 = decltype(sh2);
     int st;
     GDN_TRY_CUDA(cudaFuncSetAttribute(res::tm_res<S, S2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      220 * 1024));
+                                      int(kResSmem)));
     uint64_t k = 0;
     for (int seg0 = 0; seg0 < w.n_steps; seg0 += w.seg) {
       const int cnt = std::min(w.seg, w.n_steps - seg0);

@@ -83,6 +83,12 @@ struct RDev {
   uint4* xch;          // words in flight: [parity][NF + 2 NP][padded plane]
   const T* pv;         // [step - seg0][n_inj] injected values
   int n_inj, dft_f64;
+  // A rectangle's first val_cap injections are staged in shared memory, from
+  // element val_at on. As many as the largest rectangle holds wherever they fit:
+  // fetched from pv entry by entry instead, past a fixed 256 of them, the 360 of
+  // a rectangle that a flux contour crosses set the pace of the whole 1024 x 1024
+  // adjoint run (38.1 us a block of four steps; staged 17.8).
+  int val_at, val_cap;
   const int* vl_off;   // per rectangle CSR over vl: injections it holds
   const int* vl;       // injection index (Jz, Mx, My, ports)
   const RHdr* hdr;     // [slot][NT]
@@ -112,17 +118,16 @@ struct Shape {
   static constexpr int NW = NW_, R = R_, V = V_, NT = NW * 32;
   static constexpr int EH = NW * R, EW = 32 * V;        // extended cells
   static constexpr int TI = EH - 2 * TB, TJ = EW - 2 * TB;  // most owned cells
-  static constexpr int MAXV = 4096 / int(sizeof(T));
   static constexpr int MREG = R * V <= 8 ? 3 : 1;  // monitor parts a thread keeps in registers
   // Words of a cell: NF of fields {Ez, Hx, Hy, block} (float) or {value,
   // block} each (double); NP per psi pair (ezx, hyx), (ezy, hxy).
   static constexpr int NF = sizeof(T) == 4 ? 1 : 3, NP = sizeof(T) == 4 ? 1 : 2;
   // Dynamic shared memory, in elements: first Ez row and last Hy row of every
-  // warp, staged values, staged frame or halo cells (Ez, Hx, Hy: eight rows of
-  // EW, then eight columns of the rows between them), ca, cb; general rectangles
-  // add coefficients and psi.
+  // warp, staged frame or halo cells (Ez, Hx, Hy: eight rows of EW, then eight
+  // columns of the rows between them), ca, cb; general rectangles add
+  // coefficients and psi. The injected values of a block follow (RDev).
   static constexpr int NB = 2 * TB * (EH + EW);
-  static constexpr int O_Y = NW * EW, O_VAL = 2 * NW * EW, O_B = O_VAL + MAXV, O_C = O_B + 3 * NB;
+  static constexpr int O_Y = NW * EW, O_B = 2 * NW * EW, O_C = O_B + 3 * NB;
   static constexpr int O_GEN = O_C + 2 * EH * EW;
   using K = Coef<T, EH, EW>;
   static constexpr int KE = int((sizeof(K) + 15) / 16 * 16 / sizeof(T));
@@ -351,7 +356,7 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
       U.vb = D.vl_off[tl.idx];
       U.nv = D.vl_off[tl.idx + 1] - U.vb;
     }
-    U.nvs = min(U.nv, S::MAXV / TB);
+    U.nvs = min(U.nv, D.val_cap);
     if constexpr (GEN) {
       U.sx = slab_range(U.ie, EH, d.nx, d.npml);
       U.sy = slab_range(U.je, EW, d.ny, d.npml);
@@ -722,7 +727,7 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
       const int nvs = U.nvs, nsub = min(TB, d.n_steps - b * TB);
       for (int q = threadIdx.x; q < nvs * nsub; q += S::NT) {
         const int s = q / nvs, v = q - s * nvs;
-        sm[S::O_VAL + q] = D.pv[(long long)(b * TB + s - a.seg0) * D.n_inj + D.vl[U.vb + v]];
+        sm[D.val_at + q] = D.pv[(long long)(b * TB + s - a.seg0) * D.n_inj + D.vl[U.vb + v]];
       }
     }
     if (b == a.blk0) {
@@ -802,10 +807,10 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
       }
       // Value of injection `v` of the rectangle at this step.
       auto value = [&](int v) {
-        return v < U.nvs ? sm[S::O_VAL + (n - b * TB) * U.nvs + v]
+        return v < U.nvs ? sm[D.val_at + (n - b * TB) * U.nvs + v]
                          : D.pv[(long long)(n - a.seg0) * D.n_inj + D.vl[U.vb + v]];
       };
-      const T* const staged = sm + S::O_VAL + (n - b * TB) * U.nvs;
+      const T* const staged = sm + D.val_at + (n - b * TB) * U.nvs;
       if ((flags & 129) == 129) {  // Mx / My, one a cell at most
         const RHdr& hd = D.hdr[(long long)tl.slot * S::NT + threadIdx.x];
         const T* v = staged + hd.v_h;
