@@ -121,6 +121,11 @@ cudaStream_t capture_side_stream() {
   return streams[dev];
 }
 
+std::mutex& capture_mutex() {
+  static std::mutex mu;
+  return mu;
+}
+
 std::mutex& coop_mutex() {
   static std::mutex mu;
   return mu;

@@ -80,6 +80,9 @@ class LoopTimer {
 cudaStream_t capture_stream();
 // A second private stream per device for parallel branches inside captures.
 cudaStream_t capture_side_stream();
+// Held from the beginning to the end of a capture on those streams: threads
+// that run at the same time share them.
+std::mutex& capture_mutex();
 
 // Cooperative launches of this process on one device follow one another: the
 // lock is held while a launch waits for the event and records it anew.

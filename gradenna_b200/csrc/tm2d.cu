@@ -2361,10 +2361,12 @@ static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers*
     cudaStream_t cs = capture_stream();
     if (!cs) GDN_BAD_ARG("no capture stream for this device");
     cudaStream_t side = capture_side_stream();
+    std::unique_lock<std::mutex> lock(capture_mutex());
     GDN_TRY_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     per_chunk = enqueue_chunk(R, p, cnt, cs, side, ev_fork, ev_join);
     cudaGraph_t g = nullptr;
     const cudaError_t e1 = cudaStreamEndCapture(cs, &g);
+    lock.unlock();
     if (e1 != cudaSuccess) {
       set_error("graph capture failed: %s", cudaGetErrorString(e1));
       return GDN_ERR_CUDA;

@@ -1505,10 +1505,12 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
           if (e[q]) cudaEventDestroy(e[q]);
       }
     } ev_guard{ev};
+    std::unique_lock<std::mutex> lock(capture_mutex());
     GDN_TRY_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     *nodes = enqueue(cnt, cs, evs ? side : nullptr, ev);
     cudaGraph_t g = nullptr;
     const cudaError_t e1 = cudaStreamEndCapture(cs, &g);
+    lock.unlock();
     if (e1 != cudaSuccess) {
       set_error("graph capture failed: %s", cudaGetErrorString(e1));
       return GDN_ERR_CUDA;
