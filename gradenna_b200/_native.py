@@ -93,10 +93,11 @@ def _configure(lib) -> None:
     lib.gdn_kernel_launches.argtypes = []
     lib.gdn_tm_loop_stats.restype = ctypes.c_int
     lib.gdn_tm_loop_stats.argtypes = [P_f64, P_f64, ctypes.POINTER(ctypes.c_int64), c_int32]
-    lib.gdn_tm_workspace_size.restype = ctypes.c_int
-    lib.gdn_tm_workspace_size.argtypes = [
-        ctypes.POINTER(TmParams), ctypes.POINTER(TmPoints), ctypes.c_int,
-        ctypes.POINTER(ctypes.c_size_t)]
+    for name in ("gdn_tm_workspace_size", "gdn_tm_workspace_least"):
+        fn = getattr(lib, name)
+        fn.restype = ctypes.c_int
+        fn.argtypes = [ctypes.POINTER(TmParams), ctypes.POINTER(TmPoints), ctypes.c_int,
+                       ctypes.POINTER(ctypes.c_size_t)]
     for name in ("gdn_tm_run_f32", "gdn_tm_run_f64"):
         fn = getattr(lib, name)
         fn.restype = ctypes.c_int
@@ -167,6 +168,26 @@ def require_cuda(device=None):
 def ptr(t) -> int | None:
     """Device pointer of a tensor (None for None)."""
     return None if t is None else t.data_ptr()
+
+
+def scratch(size, least, params, points, f64, device):
+    """Device scratch of a run: what `size` (gdn_*_workspace_size) asks for, or,
+    where the memory left does not hold that, `least` (gdn_*_workspace_least)."""
+    import torch
+
+    def ask(fn):
+        n = ctypes.c_size_t(0)
+        check(fn(ctypes.byref(params), ctypes.byref(points), int(f64), ctypes.byref(n)))
+        return int(n.value)
+
+    n = ask(size)
+    try:
+        return torch.empty(max(n, 1), dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        m = ask(least)
+        if m >= n:
+            raise
+        return torch.empty(max(m, 1), dtype=torch.uint8, device=device)
 
 
 def kernel_launches() -> int:

@@ -2192,7 +2192,9 @@ struct Wave {
 
 // One cooperative launch. Tiles of two such launches wait only for their own,
 // but each needs all of its tiles on the device: launches of this process on
-// one device follow one another.
+// one device follow one another. (Three 140 x 140 runs of 3500 steps on three
+// streams take 19.9 ms; the tile kernels, whose graphs held each call back until
+// the device was idle, took 44.8.)
 template <class S, class S2>
 static int launch_coop(const res::RArgs<typename S::T>& a, int n_tiles, size_t smem,
                        cudaStream_t stream) {
@@ -2611,8 +2613,8 @@ static int run_batch_f32(const GdnTmProblem* probs, int n, int cfg, cudaStream_t
 }  // namespace tm2d
 }  // namespace gdn
 
-extern "C" int gdn_tm_workspace_size(const GdnTmParams* p, const GdnTmPoints* pts, int f64,
-                                     size_t* bytes) {
+static int tm_workspace(const GdnTmParams* p, const GdnTmPoints* pts, int f64, bool least,
+                        size_t* bytes) {
   if (!p || !bytes) {
     gdn::set_error("null argument");
     return GDN_ERR_BAD_ARG;
@@ -2627,9 +2629,20 @@ extern "C" int gdn_tm_workspace_size(const GdnTmParams* p, const GdnTmPoints* pt
   }
   // A batch runs the tile kernels on the same scratch, a single run may not.
   const size_t esize = f64 ? sizeof(double) : sizeof(float);
-  *bytes = std::max(gdn::tm2d::make_layout(p, pts, esize).total,
-                    gdn::tm2d::make_layout(p, pts, esize, 0, -1, false).total);
+  const size_t any = gdn::tm2d::make_layout(p, pts, esize).total;
+  const size_t tile = gdn::tm2d::make_layout(p, pts, esize, 0, -1, false).total;
+  *bytes = least ? std::min(any, tile) : std::max(any, tile);
   return GDN_OK;
+}
+
+extern "C" int gdn_tm_workspace_size(const GdnTmParams* p, const GdnTmPoints* pts, int f64,
+                                     size_t* bytes) {
+  return tm_workspace(p, pts, f64, false, bytes);
+}
+
+extern "C" int gdn_tm_workspace_least(const GdnTmParams* p, const GdnTmPoints* pts, int f64,
+                                      size_t* bytes) {
+  return tm_workspace(p, pts, f64, true, bytes);
 }
 
 extern "C" int gdn_tm_run_f32(const GdnTmParams* p, const GdnTmPoints* pts,

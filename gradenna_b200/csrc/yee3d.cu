@@ -1571,8 +1571,8 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
 }  // namespace yee3d
 }  // namespace gdn
 
-extern "C" int gdn_yee_workspace_size(const GdnYeeParams* p, const GdnYeePoints* pts, int f64,
-                                      size_t* bytes) {
+static int yee_workspace(const GdnYeeParams* p, const GdnYeePoints* pts, int f64, bool least,
+                         size_t* bytes) {
   if (!p || !bytes) {
     gdn::set_error("null argument");
     return GDN_ERR_BAD_ARG;
@@ -1585,8 +1585,18 @@ extern "C" int gdn_yee_workspace_size(const GdnYeeParams* p, const GdnYeePoints*
     gdn::set_error("monitor list is null");
     return GDN_ERR_BAD_ARG;
   }
-  *bytes = gdn::yee3d::make_layout3(p, pts, f64 ? sizeof(double) : sizeof(float)).total;
+  *bytes = gdn::yee3d::make_layout3(p, pts, f64 ? sizeof(double) : sizeof(float), !least).total;
   return GDN_OK;
+}
+
+extern "C" int gdn_yee_workspace_size(const GdnYeeParams* p, const GdnYeePoints* pts, int f64,
+                                      size_t* bytes) {
+  return yee_workspace(p, pts, f64, false, bytes);
+}
+
+extern "C" int gdn_yee_workspace_least(const GdnYeeParams* p, const GdnYeePoints* pts, int f64,
+                                       size_t* bytes) {
+  return yee_workspace(p, pts, f64, true, bytes);
 }
 
 extern "C" int gdn_yee_state_size(const GdnYeeParams* p, int f64, size_t* bytes) {

@@ -16,7 +16,11 @@ Two kinds of figures, in GiB:
   design-cell Ez histories of the time-domain adjoint. Gradients here need
   no reverse-mode tape: the frequency-domain adjoint keeps the forward
   design phasors during the adjoint run, the time-domain adjoint keeps two
-  n_steps x design-cell histories.
+  n_steps x design-cell histories. They count the least scratch that a run
+  takes (gdn_*_workspace_least): with memory to spare a run takes more for its
+  faster kernels (2D: 96 B a cell in float32, 224 in float64, at most 64 MiB of
+  injected values and a monitor ring of up to 256 MiB or 32 slots, whichever is
+  more; 3D: two more volumes), and does without it otherwise.
 
 All figures are first-order array sizes; leave headroom (``fits_gpu``
 defaults to 85 % of the memory).
@@ -113,7 +117,10 @@ def fdtd2d_memory_estimate(grid, n_steps: int, *, n_dft_freqs: int = 0, dtype="f
     nx, ny = grid.nx, grid.ny
     b = _itemsize(dtype)
     acc = _itemsize(dft_dtype) if dft_dtype is not None else 2 * b
-    plane = (nx + 16) * (ny + 64)
+    # whole tiles: small grids are cut into 16 x 32 cells, others into 32 (16) x 64
+    big = -(-nx // (64 if b == 4 else 28)) * -(-ny // 64) >= 148
+    ti, tj = (32 if b == 4 else 16, 64) if big else (16, 32)
+    plane = (-(-nx // ti) * ti + 16) * (-(-ny // tj) * tj + 64)
     # 2 slots x (Ez, Hx, Hy, 4 psi) + ca, cb
     planes = (2 * 7 + 2) * plane * b
     mon = (3 * nx * ny) if monitor_cells is None else int(monitor_cells)

@@ -532,11 +532,9 @@ def simulate_tm(
     """
     p = _prepare_tm(grid, source_ij=source_ij, source_current=source_current, eps_r=eps_r, sigma=sigma, probe_ij=probe_ij, ports=ports, dft_freqs=dft_freqs, dft_dtype=dft_dtype, cpml=cpml, record_energy=record_energy, mx_ij=mx_ij, mx_current=mx_current, my_ij=my_ij, my_current=my_current, dtype=dtype, device=device, dft_region=dft_region, dft_monitors=dft_monitors, cw_sources=cw_sources)
     lib = _native.load()
-    nbytes = ctypes.c_size_t(0)
-    _native.check(lib.gdn_tm_workspace_size(ctypes.byref(p.params), ctypes.byref(p.pts),
-                                            int(p.f64), ctypes.byref(nbytes)))
-    ws = torch.empty(max(int(nbytes.value), 1), dtype=torch.uint8, device=p.dev)
-    p.bufs.workspace, p.bufs.workspace_bytes = ws.data_ptr(), int(nbytes.value)
+    ws = _native.scratch(lib.gdn_tm_workspace_size, lib.gdn_tm_workspace_least, p.params, p.pts,
+                         p.f64, p.dev)
+    p.bufs.workspace, p.bufs.workspace_bytes = ws.data_ptr(), ws.numel()
     stream = torch.cuda.current_stream(p.dev)
     run = lib.gdn_tm_run_f64 if p.f64 else lib.gdn_tm_run_f32
     with torch.cuda.device(p.dev):

@@ -130,9 +130,9 @@ class YeeBuffers(ctypes.Structure):
                    ("state_in", V), ("state_out", V)])
 
 
-_native.register("gdn_yee_workspace_size", ctypes.c_int, [
-    ctypes.POINTER(YeeParams), ctypes.POINTER(YeePoints), ctypes.c_int,
-    ctypes.POINTER(ctypes.c_size_t)])
+for _name in ("gdn_yee_workspace_size", "gdn_yee_workspace_least"):
+    _native.register(_name, ctypes.c_int, [ctypes.POINTER(YeeParams), ctypes.POINTER(YeePoints),
+                                           ctypes.c_int, ctypes.POINTER(ctypes.c_size_t)])
 _native.register("gdn_yee_state_size", ctypes.c_int, [
     ctypes.POINTER(YeeParams), ctypes.c_int, ctypes.POINTER(ctypes.c_size_t)])
 for _name in ("gdn_yee_run_f32", "gdn_yee_run_f64"):
@@ -452,11 +452,9 @@ def simulate_3d(
             bufs.dft[c] = mon_out[c].data_ptr()
 
     f64 = fdt == torch.float64
-    nbytes = ctypes.c_size_t(0)
-    _native.check(lib.gdn_yee_workspace_size(ctypes.byref(prm), ctypes.byref(pts), int(f64),
-                                             ctypes.byref(nbytes)))
-    ws = torch.empty(max(int(nbytes.value), 1), dtype=torch.uint8, device=dev)
-    bufs.workspace, bufs.workspace_bytes = ws.data_ptr(), int(nbytes.value)
+    ws = _native.scratch(lib.gdn_yee_workspace_size, lib.gdn_yee_workspace_least, prm, pts, f64,
+                         dev)
+    bufs.workspace, bufs.workspace_bytes = ws.data_ptr(), ws.numel()
     state_out = None
     if state_in is not None or return_state:
         sbytes = ctypes.c_size_t(0)

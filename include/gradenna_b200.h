@@ -167,6 +167,11 @@ typedef struct GdnTmBuffers {
  * monitors). */
 int gdn_tm_workspace_size(const GdnTmParams* p, const GdnTmPoints* pts, int f64, size_t* bytes);
 
+/* The least scratch gdn_tm_run_* takes instead, for callers that are short of
+ * memory: the same results from kernels that are slower where the two sizes
+ * differ. */
+int gdn_tm_workspace_least(const GdnTmParams* p, const GdnTmPoints* pts, int f64, size_t* bytes);
+
 /* Run the whole 2D TM time loop (replaces gradenna_tm_run_f32/_f64,
  * rust/src/lib.rs:89-641). Stream-ordered; host index lists are consumed
  * before return. */
@@ -310,6 +315,8 @@ typedef struct GdnYeeBuffers {
 } GdnYeeBuffers;
 
 int gdn_yee_workspace_size(const GdnYeeParams* p, const GdnYeePoints* pts, int f64, size_t* bytes);
+/* The least scratch gdn_yee_run_* takes instead (same results, slower). */
+int gdn_yee_workspace_least(const GdnYeeParams* p, const GdnYeePoints* pts, int f64, size_t* bytes);
 
 /* Bytes of the resumable state blob of a grid (see GdnYeeBuffers.state_in). */
 int gdn_yee_state_size(const GdnYeeParams* p, int f64, size_t* bytes);
