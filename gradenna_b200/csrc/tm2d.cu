@@ -2295,6 +2295,13 @@ static int refuse_capture(cudaStream_t stream) {
   return GDN_OK;
 }
 
+// The caller's scratch, or null where the run takes its own: every kernel moves
+// 16 bytes at a time, on 16-byte boundaries.
+static char* usable_scratch(const GdnTmBuffers* b) {
+  char* ws = static_cast<char*>(b->workspace);
+  return reinterpret_cast<uintptr_t>(ws) % 16 ? nullptr : ws;
+}
+
 template <typename T>
 static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers* b,
                cudaStream_t stream) {
@@ -2304,12 +2311,10 @@ static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers*
   Run<T> R;
   R.L = make_layout(p, pts, sizeof(T));
   if (R.L.res && (st = refuse_capture(stream))) return st;
-  char* ws = static_cast<char*>(b->workspace);
+  char* ws = usable_scratch(b);
   bool own = false;
-  // Scratch that holds the tile kernels' layout only, or off the 16-byte
-  // boundaries that the exchanged words need, is enough for them.
-  if (ws && R.L.res &&
-      (b->workspace_bytes < R.L.total || reinterpret_cast<uintptr_t>(ws) % 16))
+  // Scratch that holds the tile kernels' layout only is enough for them.
+  if (ws && R.L.res && b->workspace_bytes < R.L.total)
     R.L = make_layout(p, pts, sizeof(T), 0, -1, false);
   if (!ws) {
     cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ws), R.L.total, stream);
@@ -2483,7 +2488,7 @@ static int run_batch_f32(const GdnTmProblem* probs, int n, int cfg, cudaStream_t
     if (R[q].L.R != ring)
       R[q].L = make_layout(probs[q].params, probs[q].points, sizeof(T), ring, which, false);
     const GdnTmBuffers* b = probs[q].buffers;
-    if (b->workspace) {
+    if (usable_scratch(b)) {
       if (b->workspace_bytes < R[q].L.total)
         GDN_BAD_ARG("problem %d: workspace too small: %zu < %zu bytes", q, b->workspace_bytes,
                     R[q].L.total);
@@ -2531,7 +2536,7 @@ static int run_batch_f32(const GdnTmProblem* probs, int n, int cfg, cudaStream_t
   std::vector<Dev<T>> hdev(n);
   for (int q = 0; q < n; ++q) {
     const GdnTmBuffers* b = probs[q].buffers;
-    char* ws = b->workspace ? static_cast<char*>(b->workspace) : block + woff[q];
+    char* ws = usable_scratch(b) ? usable_scratch(b) : block + woff[q];
     if ((st = prepare(probs[q].params, probs[q].points, b, ws, R[q], stream))) {
       const std::string msg = last_error();
       GDN_BAD_ARG("problem %d: %s", q, msg.c_str());

@@ -31,7 +31,8 @@
  *     be read back (documented per entry point).
  *   - The caller owns every buffer. Scratch: pass `workspace` of at least
  *     gdn_*_workspace_size() bytes, or NULL to let the library allocate it
- *     stream-ordered for the duration of the call.
+ *     stream-ordered for the duration of the call. Scratch that does not start
+ *     on a 16-byte boundary is treated as NULL.
  */
 #ifndef GRADENNA_B200_H
 #define GRADENNA_B200_H
