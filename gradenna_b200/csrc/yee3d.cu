@@ -1097,8 +1097,8 @@ static int validate3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYe
 
 // Launch with programmatic stream serialisation (see dependent_launch_gate).
 template <typename... KArgs, typename... Args>
-static void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
-                       Args... args) {
+static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
+                              Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -1109,11 +1109,12 @@ static void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStre
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // Planes per CTA for a step kernel: as few as let every CTA of the `cols`
-// column blocks be resident at once, two at most. Each plane is a trip to L2
+// column blocks be resident at once, two at most (more only where the planes
+// would be too many for a grid's second extent). Each plane is a trip to L2
 // that only other warps hide: at 160 x 160 x 64 f32 a step with 7 planes a CTA
 // (one wave) takes 53 us, with two (three waves) 50, with one 54; at 97 x 83 x
 // 61 four planes instead of two cost a quarter more.
@@ -1126,6 +1127,7 @@ static int planes_per_cta(K kernel, int nx, int cols, int* ni) {
   const long long slots = (long long)std::max(sms, 1) * std::max(per_sm, 1);
   const long long per_col = std::max<long long>(1, slots / std::max(cols, 1));
   *ni = int(std::min<long long>(2, std::max<long long>(1, div_up(nx, per_col))));
+  *ni = int(std::max<long long>(*ni, div_up(nx, 65535)));
   return GDN_OK;
 }
 
@@ -1413,8 +1415,6 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
   }
 
   const dim3 blk(NT);
-  // Planes per CTA: the fewest that fit every CTA of the grid into one wave
-  // of resident CTAs (a partial second wave would idle most SMs).
   int ni_h = 0, ni_e = 0;
   if ((st = planes_per_cta(yee_h<T>, nx, L.cols, &ni_h))) return st;
   if ((st = planes_per_cta(yee_e<T>, nx, L.cols, &ni_e))) return st;
@@ -1426,8 +1426,13 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
   // step t overlaps yee_e of step t and the E gather overlaps yee_h of step
   // t + 1; each field's next writer waits for its gather (events), and the
   // fold waits for the last ones.
+  cudaError_t launch_err = cudaSuccess;  // of a chunk's step and injection kernels
   auto enqueue = [&](int cnt, cudaStream_t s, cudaStream_t side, cudaEvent_t* ev) -> uint64_t {
     uint64_t k = 0;
+    auto launch = [&](auto kernel, dim3 grid, dim3 block, cudaStream_t st_, auto... args) {
+      const cudaError_t e = launch_pdl(kernel, grid, block, st_, args...);
+      if (launch_err == cudaSuccess) launch_err = e;
+    };
     bool pend_h = false, pend_e = false;  // a gather still reads H / E
     auto gather = [&](int t, int sd, unsigned blocks) {
       if (!side) {
@@ -1452,10 +1457,10 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
     const unsigned gb0 = unsigned(div_up(d.gcells[0], 256)), gb1 = unsigned(div_up(d.gcells[1], 256));
     for (int t = 0; t < cnt; ++t) {
       settle(pend_h, 1);
-      launch_pdl(yee_h<T>, grd_h, blk, s, d, ni_h);
+      launch(yee_h<T>, grd_h, blk, s, d, ni_h);
       k += 1;
       if (d.n_fp[1] > 0) {
-        launch_pdl(yee_inject<T>, dim3(unsigned(div_up(d.n_fp[1], 256))), dim3(256), s, d, t, 1);
+        launch(yee_inject<T>, dim3(unsigned(div_up(d.n_fp[1], 256))), dim3(256), s, d, t, 1);
         ++k;
       }
       if (gb1 > 0) {
@@ -1463,10 +1468,10 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
         ++k;
       }
       settle(pend_e, 0);
-      launch_pdl(yee_e<T>, grd_e, blk, s, d, t, ni_e);
+      launch(yee_e<T>, grd_e, blk, s, d, t, ni_e);
       k += 1;
       if (d.n_fp[0] > 0) {
-        launch_pdl(yee_inject<T>, dim3(unsigned(div_up(d.n_fp[0], 256))), dim3(256), s, d, t, 0);
+        launch(yee_inject<T>, dim3(unsigned(div_up(d.n_fp[0], 256))), dim3(256), s, d, t, 0);
         ++k;
       }
       if (gb0 > 0) {
@@ -1507,10 +1512,17 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
     } ev_guard{ev};
     std::unique_lock<std::mutex> lock(capture_mutex());
     GDN_TRY_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+    launch_err = cudaSuccess;
     *nodes = enqueue(cnt, cs, evs ? side : nullptr, ev);
     cudaGraph_t g = nullptr;
-    const cudaError_t e1 = cudaStreamEndCapture(cs, &g);
+    cudaError_t e1 = cudaStreamEndCapture(cs, &g);
     lock.unlock();
+    if (e1 == cudaSuccess && launch_err != cudaSuccess) {
+      // A graph without one of its kernels is not run.
+      cudaGetLastError();
+      cudaGraphDestroy(g);
+      e1 = launch_err;
+    }
     if (e1 != cudaSuccess) {
       set_error("graph capture failed: %s", cudaGetErrorString(e1));
       return GDN_ERR_CUDA;
