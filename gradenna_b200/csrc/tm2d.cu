@@ -2220,25 +2220,16 @@ static int launch_coop(const res::RArgs<typename S::T>& a, int n_tiles, size_t s
   return GDN_OK;
 }
 
-template <typename T, typename A, int KM, int NC>
-static void launch_seg_fold_nc(const Wave<T>& w, int seg0, cudaStream_t s) {
-  const dim3 grid(unsigned(div_up(w.mon_max, 256 * NC)), unsigned(w.n_prob));
-  const size_t sm = size_t(4) * res::FOLD * w.kmax * sizeof(A);
-  res::tm_seg_fold<T, A, KM, NC><<<grid, 256, sm, s>>>(w.devs, seg0, w.seg);
-}
-
-// Cells per thread: as many as the accumulators leave registers for, and one
-// where few cells would leave SMs idle.
 template <typename T, typename A>
-static void launch_seg_fold(const Wave<T>& w, int seg0, cudaStream_t s) {
-  constexpr bool wide = sizeof(A) == 8;
-  const bool few = w.mon_max < 148 * 1024;
+static void launch_seg_fold(const Wave<T>& w, const Dev<T>& d, int seg0, cudaStream_t s) {
+  const unsigned grid = unsigned(div_up(w.mon_max, 256));
+  const size_t sm = size_t(4) * res::FOLD * w.kmax * sizeof(A);
   if (w.kmax <= 4)
-    few ? launch_seg_fold_nc<T, A, 4, 1>(w, seg0, s) : launch_seg_fold_nc<T, A, 4, wide ? 1 : 4>(w, seg0, s);
+    res::tm_seg_fold<T, A, 4><<<grid, 256, sm, s>>>(d, seg0, w.seg);
   else if (w.kmax <= 8)
-    few ? launch_seg_fold_nc<T, A, 8, 1>(w, seg0, s) : launch_seg_fold_nc<T, A, 8, wide ? 1 : 2>(w, seg0, s);
+    res::tm_seg_fold<T, A, 8><<<grid, 256, sm, s>>>(d, seg0, w.seg);
   else
-    launch_seg_fold_nc<T, A, KMAX, 1>(w, seg0, s);
+    res::tm_seg_fold<T, A, KMAX><<<grid, 256, sm, s>>>(d, seg0, w.seg);
 }
 
 // Tests: the block whose words rectangle 0 keeps back in resident runs that this
@@ -2250,7 +2241,7 @@ constexpr int kHoldPolls = 1 << 12;  // then a few milliseconds of polls
 // cooperative launch when they all fit, else one launch per block) and the
 // DFT sums.
 template <typename T>
-static int run_wave(const Wave<T>& w, cudaStream_t stream) {
+static int run_wave(const Wave<T>& w, const Dev<T>& d, cudaStream_t stream) {
   return with_kind<T>(w.kind, [&](auto sh, auto sh2) -> int {
     using S = decltype(sh);
     using S2 = decltype(sh2);
@@ -2269,8 +2260,8 @@ static int run_wave(const Wave<T>& w, cudaStream_t stream) {
       res::RArgs<T> a{w.devs, w.tiles, w.err, b0, b1, seg0, t_hold < 0 ? res::POLLS : kHoldPolls, t_hold};
       if ((st = launch_coop<S, S2>(a, w.n_tiles, w.smem, stream))) return st;
       ++k;
-      if (w.f64) launch_seg_fold<T, double>(w, seg0, stream);
-      if (w.f32) launch_seg_fold<T, float>(w, seg0, stream);
+      if (w.f64) launch_seg_fold<T, double>(w, d, seg0, stream);
+      if (w.f32) launch_seg_fold<T, float>(w, d, seg0, stream);
       k += int(w.f64) + int(w.f32);
     }
     const cudaError_t le = cudaGetLastError();
@@ -2346,7 +2337,7 @@ static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers*
     w.kind = R.L.kind;
     w.seg = R.L.seg;
     LoopTimer timer(stream, double(p->nx) * p->ny * p->n_steps, div_up(p->n_steps, res::TB));
-    st = run_wave(w, stream);
+    st = run_wave(w, R.d, stream);
     timer.stop(st == GDN_OK);
     return st ? st : finalize(p, b, R, stream);
   }

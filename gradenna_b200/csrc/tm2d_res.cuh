@@ -1115,56 +1115,57 @@ __global__ void __launch_bounds__(128) tm_values(const RDev<T>* devs, int seg0, 
   }
 }
 
+// CTAs an SM that tm_seg_fold is compiled for: as many as its registers allow
+// without spills (more waits are hidden; see the figures at the kernel).
+template <typename T, typename A>
+constexpr int fold_ctas(int km) {
+  if (km <= 4) return sizeof(T) == 4 ? 4 : 3;
+  if (km <= 8) return sizeof(A) == 8 ? 2 : (sizeof(T) == 4 ? 4 : 3);
+  return sizeof(T) == 8 && sizeof(A) == 8 ? 1 : 2;
+}
+
 // Running DFT of a segment: per monitored cell and FOLD steps one partial sum
 // in A, added to the accumulator (the sums and their order are tm_dft_fold's).
-// A thread takes NC cells, blockDim apart, so that a phase factor read from
-// shared memory serves NC cells: with one the kernel is bound by those reads.
-template <typename T, typename A, int KM, int NC>
-__global__ void __launch_bounds__(256) tm_seg_fold(const RDev<T>* devs, int seg0, int seg) {
+// One thread a cell; the next eight samples come while eight are summed. The
+// accumulators are read and written once per FOLD steps: kept in registers for
+// the segment, beside the partial sums, they left one CTA an SM, and several
+// cells a thread did not make up for it. Bound by the ring's bytes for few tones
+// and by the multiply-adds for many. us for a ring of about 256 MB (of 32 steps
+// at 1024 x 1024), kept in registers -> here (tm_dft_fold, 32 steps a launch):
+//   full grid 140 x 140, 1024 steps, 8 tones, float samples and sums  329 -> 207 (463)
+//   400 x 400, 128 steps, 8 tones, float, float                       249 -> 136 (223)
+//   400 x 400, 128 steps, 16 tones, float, double                    1511 -> 474 (950)
+//   400 x 400, 64 steps, 8 tones, double, double                      253 -> 137 (162)
+//   1024 x 1024, 32 steps, 4 tones, float, float                      329 -> 165 (191)
+//   1024 x 1024, 32 steps, 16 tones, float, float                     726 -> 687 (587)
+template <typename T, typename A, int KM>
+__global__ void __launch_bounds__(256, fold_ctas<T, A>(KM))
+    tm_seg_fold(Dev<T> d, int seg0, int seg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using C = typename Cplx<A>::type;
   C* const sph = reinterpret_cast<C*>(smem_raw);  // [2 tables][FOLD][K]
-  const Dev<T>& d = devs[blockIdx.y].d;
   const int K = d.n_freq, total = min(seg, d.n_steps - seg0);
-  const long long r0 = (long long)blockIdx.x * blockDim.x * NC + threadIdx.x;
-  if (devs[blockIdx.y].dft_f64 != int(sizeof(A) == 8) || total <= 0 || d.n_mons == 0 ||
-      (long long)blockIdx.x * blockDim.x * NC >= d.mon_cells)
-    return;
-  C* acc[NC];
-  long long count[NC];
-  bool live[NC];
-  int tab[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const long long r = r0 + c * blockDim.x;
-    int lo = 0, hi = d.n_mons - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (d.mons[mid].off <= r)
-        lo = mid;
-      else
-        hi = mid - 1;
-    }
-    const MonD mon = d.mons[lo];
-    const long long loc = r - mon.off;
-    const int row = int(loc / mon.pitch), col = int(loc - (long long)row * mon.pitch) - mon.pad;
-    live[c] = r < d.mon_cells && row < mon.h && col >= 0 && col < mon.w;
-    acc[c] = static_cast<C*>(mon.out) + ((long long)row * mon.w + col);
-    count[c] = mon.count;
-    tab[c] = mon.comp == 0 ? 0 : FOLD * K;
+  const int r = int(blockIdx.x) * 256 + int(threadIdx.x);  // a ring slot holds < 2^31 cells
+  int lo = 0, hi = d.n_mons - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (d.mons[mid].off <= r)
+      lo = mid;
+    else
+      hi = mid - 1;
   }
-  C sum[NC][KM];
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-#pragma unroll
-    for (int k = 0; k < KM; ++k)
-      if (k < K && live[c]) sum[c][k] = acc[c][(long long)k * count[c]];
-  const T* const ring = d.mring + r0;
-  const long long stride = d.mon_cells;
+  const MonD mon = d.mons[lo];
+  const unsigned loc = unsigned(r - int(mon.off));
+  const int row = int(loc / unsigned(mon.pitch));
+  const int col = int(loc - unsigned(row) * unsigned(mon.pitch)) - mon.pad;
+  const bool live = r < d.mon_cells && row < mon.h && col >= 0 && col < mon.w;
+  C* const acc = static_cast<C*>(mon.out) + ((long long)row * mon.w + col);
+  const int tab = mon.comp == 0 ? 0 : FOLD * K;
+  const T* const ring = d.mring + r;
   for (int b0 = 0; b0 < total; b0 += FOLD) {
     const int cnt = min(FOLD, total - b0);
     __syncthreads();
-    for (int q = threadIdx.x; q < cnt * K; q += blockDim.x) {
+    for (int q = threadIdx.x; q < cnt * K; q += 256) {
       const double2 pe = d.ph_e[(long long)(seg0 + b0) * K + q];
       const double2 ph = d.ph_h[(long long)(seg0 + b0) * K + q];
       sph[q].x = A(pe.x);
@@ -1173,63 +1174,44 @@ __global__ void __launch_bounds__(256) tm_seg_fold(const RDev<T>* devs, int seg0
       sph[FOLD * K + q].y = A(ph.y);
     }
     __syncthreads();
-    C part[NC][KM];
+    if (!live) continue;
+    C part[KM];
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
+    for (int k = 0; k < KM; ++k) part[k].x = part[k].y = A(0);
+    const T* const base = ring + b0 * d.mon_cells;
+    T x[8], next[8];
+    auto fetch = [&](T (&v)[8], int t0) {
 #pragma unroll
-      for (int k = 0; k < KM; ++k) part[c][k].x = part[c][k].y = A(0);
-    const T* const base = ring + (long long)b0 * stride;
-    bool same = true;
-#pragma unroll
-    for (int c = 1; c < NC; ++c) same = same && tab[c] == tab[0];
-    T x[NC][8], next[NC][8];
-    auto fetch = [&](T (&v)[NC][8], int t0) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-          v[c][u] = live[c] && t0 + u < cnt ? base[(long long)(t0 + u) * stride + c * 256] : T(0);
+      for (int u = 0; u < 8; ++u) v[u] = t0 + u < cnt ? base[(t0 + u) * d.mon_cells] : T(0);
     };
     fetch(next, 0);
     for (int t0 = 0; t0 < cnt; t0 += 8) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int c = 0; c < NC; ++c) x[c][u] = next[c][u];
-      if (t0 + 8 < cnt) fetch(next, t0 + 8);  // the next samples come while these are summed
+      for (int u = 0; u < 8; ++u) x[u] = next[u];
+      if (t0 + 8 < cnt) fetch(next, t0 + 8);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         if (t0 + u < cnt) {
-          const C* const p0 = sph + tab[0] + (t0 + u) * K;
+          const C* const p0 = sph + tab + (t0 + u) * K;
 #pragma unroll
-          for (int k = 0; k < KM; ++k) {
+          for (int k = 0; k < KM; ++k)
             if (k < K) {
               const C p = p0[k];
-#pragma unroll
-              for (int c = 0; c < NC; ++c) {
-                const C q = same ? p : sph[tab[c] + (t0 + u) * K + k];
-                part[c][k].x += q.x * A(x[c][u]);
-                part[c][k].y += q.y * A(x[c][u]);
-              }
+              part[k].x += p.x * A(x[u]);
+              part[k].y += p.y * A(x[u]);
             }
-          }
         }
       }
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int k = 0; k < KM; ++k)
-        if (k < K) {
-          sum[c][k].x += part[c][k].x;
-          sum[c][k].y += part[c][k].y;
-        }
-  }
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-#pragma unroll
     for (int k = 0; k < KM; ++k)
-      if (k < K && live[c]) acc[c][(long long)k * count[c]] = sum[c][k];
+      if (k < K) {
+        C v = acc[(long long)k * mon.count];
+        v.x += part[k].x;
+        v.y += part[k].y;
+        acc[(long long)k * mon.count] = v;
+      }
+  }
 }
 
 }  // namespace res
