@@ -2222,14 +2222,17 @@ static int launch_coop(const res::RArgs<typename S::T>& a, int n_tiles, size_t s
 
 template <typename T, typename A>
 static void launch_seg_fold(const Wave<T>& w, const Dev<T>& d, int seg0, cudaStream_t s) {
-  const unsigned grid = unsigned(div_up(w.mon_max, 256));
   const size_t sm = size_t(4) * res::FOLD * w.kmax * sizeof(A);
+  auto launch = [&](auto km) {
+    constexpr int KM = decltype(km)::value, NT = res::fold_threads<T, A>(KM);
+    res::tm_seg_fold<T, A, KM><<<unsigned(div_up(w.mon_max, NT)), NT, sm, s>>>(d, seg0, w.seg);
+  };
   if (w.kmax <= 4)
-    res::tm_seg_fold<T, A, 4><<<grid, 256, sm, s>>>(d, seg0, w.seg);
+    launch(std::integral_constant<int, 4>{});
   else if (w.kmax <= 8)
-    res::tm_seg_fold<T, A, 8><<<grid, 256, sm, s>>>(d, seg0, w.seg);
+    launch(std::integral_constant<int, 8>{});
   else
-    res::tm_seg_fold<T, A, KMAX><<<grid, 256, sm, s>>>(d, seg0, w.seg);
+    launch(std::integral_constant<int, KMAX>{});
 }
 
 // Tests: the block whose words rectangle 0 keeps back in resident runs that this

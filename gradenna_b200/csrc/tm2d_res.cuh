@@ -1115,12 +1115,17 @@ __global__ void __launch_bounds__(128) tm_values(const RDev<T>* devs, int seg0, 
   }
 }
 
-// CTAs an SM that tm_seg_fold is compiled for: as many as its registers allow
-// without spills (more waits are hidden; see the figures at the kernel).
+// Threads of a CTA of tm_seg_fold, and CTAs an SM that it is compiled for: as
+// many as its registers allow without spills, in steps of 128 threads where 256
+// are too coarse (more waits are hidden; see the figures at the kernel).
+template <typename T, typename A>
+constexpr int fold_threads(int km) {
+  return (km == 8 && sizeof(A) == 8) || (km == 16 && sizeof(T) == 4 && sizeof(A) == 4) ? 128 : 256;
+}
 template <typename T, typename A>
 constexpr int fold_ctas(int km) {
-  if (km <= 4) return sizeof(T) == 4 ? 4 : 3;
-  if (km <= 8) return sizeof(A) == 8 ? 2 : (sizeof(T) == 4 ? 4 : 3);
+  if (fold_threads<T, A>(km) == 128) return 5;
+  if (km <= 8) return sizeof(T) == 4 ? 4 : 3;
   return sizeof(T) == 8 && sizeof(A) == 8 ? 1 : 2;
 }
 
@@ -1135,17 +1140,18 @@ constexpr int fold_ctas(int km) {
 //   full grid 140 x 140, 1024 steps, 8 tones, float samples and sums  329 -> 207 (463)
 //   400 x 400, 128 steps, 8 tones, float, float                       249 -> 136 (223)
 //   400 x 400, 128 steps, 16 tones, float, double                    1511 -> 474 (950)
-//   400 x 400, 64 steps, 8 tones, double, double                      253 -> 137 (162)
+//   400 x 400, 64 steps, 8 tones, double, double                      253 -> 123 (159)
 //   1024 x 1024, 32 steps, 4 tones, float, float                      329 -> 165 (191)
-//   1024 x 1024, 32 steps, 16 tones, float, float                     726 -> 687 (587)
+//   1024 x 1024, 32 steps, 16 tones, float, float                     726 -> 560 (576)
 template <typename T, typename A, int KM>
-__global__ void __launch_bounds__(256, fold_ctas<T, A>(KM))
+__global__ void __launch_bounds__(fold_threads<T, A>(KM), fold_ctas<T, A>(KM))
     tm_seg_fold(Dev<T> d, int seg0, int seg) {
+  constexpr int NT = fold_threads<T, A>(KM);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using C = typename Cplx<A>::type;
   C* const sph = reinterpret_cast<C*>(smem_raw);  // [2 tables][FOLD][K]
   const int K = d.n_freq, total = min(seg, d.n_steps - seg0);
-  const int r = int(blockIdx.x) * 256 + int(threadIdx.x);  // a ring slot holds < 2^31 cells
+  const int r = int(blockIdx.x) * NT + int(threadIdx.x);  // a ring slot holds < 2^31 cells
   int lo = 0, hi = d.n_mons - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -1165,7 +1171,7 @@ __global__ void __launch_bounds__(256, fold_ctas<T, A>(KM))
   for (int b0 = 0; b0 < total; b0 += FOLD) {
     const int cnt = min(FOLD, total - b0);
     __syncthreads();
-    for (int q = threadIdx.x; q < cnt * K; q += 256) {
+    for (int q = threadIdx.x; q < cnt * K; q += NT) {
       const double2 pe = d.ph_e[(long long)(seg0 + b0) * K + q];
       const double2 ph = d.ph_h[(long long)(seg0 + b0) * K + q];
       sph[q].x = A(pe.x);
