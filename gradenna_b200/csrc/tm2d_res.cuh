@@ -1032,10 +1032,16 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
 #pragma unroll
             for (int r = 0; r < R; ++r)
               if (r >= lo && r < hi) {
+                T v[V];
 #pragma unroll
-                for (int k = 0; k < V; ++k)
-                  if (cm >> k & 1)
-                    o[r * w.w + k] = w.comp == 0 ? e[r][k] : (w.comp == 1 ? hx[r][k] : hy[r][k]);
+                for (int k = 0; k < V; ++k) v[k] = w.comp == 0 ? e[r][k] : (w.comp == 1 ? hx[r][k] : hy[r][k]);
+                if (cm == (1u << V) - 1) {
+                  sts(o + r * w.w, v);
+                } else {
+#pragma unroll
+                  for (int k = 0; k < V; ++k)
+                    if (cm >> k & 1) o[r * w.w + k] = v[k];
+                }
               }
           };
           for (unsigned mk = pmask; mk; mk &= mk - 1) {

@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 CASES = [(517, 4, torch.float32, np.complex64), (517, 8, torch.float32, np.complex64),
          (400, 16, torch.float32, np.complex128), (1024, 16, torch.float32, np.complex128),
          (400, 9, torch.float64, np.complex64), (400, 16, torch.float64, np.complex128),
-         (280, 5, torch.float64, np.complex128), (140, 16, torch.float32, np.complex64)]
+         (280, 5, torch.float64, np.complex128), (140, 16, torch.float32, np.complex64),
+         (640, 1, torch.float32, np.complex64), (1024, 4, torch.float32, np.complex64)]
 
 
 @pytest.mark.parametrize("n,tones,dtype,cdtype", CASES)
