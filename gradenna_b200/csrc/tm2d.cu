@@ -1101,6 +1101,24 @@ static res::Rect rect_at(const Region& g, int r, int q) {
   return res::Rect{i0, j0, std::min(g.ph, g.i0 + g.h - i0), std::min(g.pw, g.j0 + g.w - j0), g.gen};
 }
 
+// Whether a rectangle holds so many probes that reading them off sets its pace:
+// its 512 threads store them one by one, and all others wait. Only the large
+// rectangles of float kinds D and E hold that many. Time loops of 400 steps at
+// 640 x 640 (300 at 1024 x 1024), resident against tile kernels, ms: a block of
+// 40 x 40 probes 1.35 : 1.73 (1.46 : 1.90), 100 x 100, of which a rectangle
+// holds 5300 (5000), 2.20 : 1.72 (1.75 : 1.94), 200 x 200, which fill
+// rectangles, 2.43 : 1.73 (2.32 : 2.00).
+constexpr int kCrowd = 4096;
+static bool crowded(const Plan& pl, const GdnTmParams* p, const GdnTmPoints* pts) {
+  if (p->n_probes <= kCrowd || !pts || !pts->probe_i || !pts->probe_j) return false;
+  std::vector<int> n(size_t(pl.n_rects), 0);
+  for (int m = 0; m < p->n_probes; ++m) {
+    const int i = pts->probe_i[m], j = pts->probe_j[m];
+    rects_of(pl, i, i + 1, j, j + 1, [&](const Region&, int, int, int idx) { ++n[size_t(idx)]; });
+  }
+  return *std::max_element(n.begin(), n.end()) > kCrowd;
+}
+
 // Bound on the copies of points in rectangles and their halos.
 static size_t res_copies(const Plan& pl, const GdnTmParams* p) {
   const size_t np = size_t(p->n_sources) + p->n_mx + p->n_my + p->n_ports;
@@ -1136,7 +1154,7 @@ static Layout make_layout(const GdnTmParams* p, const GdnTmPoints* pts, size_t e
     L.res = use_res(p, pts, esize, c);
     if (L.res) {
       L.kind = choose_kind(p, esize, c, &L.plan);
-      L.res = L.kind >= 0;
+      L.res = L.kind >= 0 && !crowded(L.plan, p, pts);
     }
   }
   L.cfg = L.march ? (esize == sizeof(float) ? march_cfg<float>() : march_cfg<double>())
@@ -2121,6 +2139,10 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
               }
             }
           }
+          // Probes by register (a kernel reads them off in that order where no
+          // register has two).
+          std::sort(x0 + n_mag + n_jz + n_port, x0 + n_mag + n_jz + n_port + int(h.n23 >> 16),
+                    [](const res::RPt& u, const res::RPt& v) { return u.reg() < v.reg(); });
           for (int q = 0; q < n_port; ++q) {
             res::RPt& e = x0[n_mag + n_jz + q];
             for (const auto& pv : port_val)

@@ -56,7 +56,7 @@ struct Rect {
 // register r * V + k (8 bits), kind (2 bits: 0 Hx, 1 Hy for magnetic currents; 1
 // = owner for ports) and the index of its value among the rectangle's
 // injections (22 bits; a port's is also its number in the rectangle).
-struct RPt {
+struct __align__(8) RPt {
   int m;
   unsigned w;
   __host__ __device__ int reg() const { return int(w & 255); }
@@ -410,17 +410,37 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
              (n23 >> 16 ? 8u : 0u) | hd.dense << 7;
   }
   // Entry q of this thread's list; begin and end of a class in it.
-  auto entry = [&](int q) { return q < MAXE ? U.pts[q] : D.pts[U.pb + q]; };
+  auto entry = [&](int q) {
+    if (q < MAXE) return U.pts[q];
+    const int2 p = __ldg(reinterpret_cast<const int2*>(D.pts + U.pb + q));
+    return RPt{p.x, unsigned(p.y)};
+  };
   auto at_jz = [&]() { return hd_first + int(n01 & 0xffff); };
   auto at_port = [&]() { return at_jz() + int(n01 >> 16); };
   auto at_probe = [&]() { return at_port() + int(n23 & 0xffff); };
   auto at_end = [&]() { return at_probe() + int(n23 >> 16); };
   if (__any_sync(0xffffffffu, flags & 4)) flags |= 32;
-  int probe = -1;  // a thread's only probe: its index, register in bits 24 .. 31 of flags
+  // Probes: of a thread's only one its index, and its register in bits 24 .. 31 of
+  // flags; of several in as many registers (flag 512) the mask of these.
+  int probe = -1;
   if ((flags & 8) && n23 >> 16 == 1) {
     const RPt q = entry(at_probe());
     probe = q.m;
     flags |= unsigned(q.reg()) << 24;
+  } else if (flags & 8) {
+    unsigned mask = 0;
+    int last = -1;
+    bool once = true;
+    for (int q = at_probe(); q < at_end(); ++q) {
+      const int reg = entry(q).reg();
+      once = once && reg > last && reg < 32;
+      mask |= 1u << (reg & 31);
+      last = reg;
+    }
+    if (once) {
+      flags |= 512;
+      probe = int(mask);
+    }
   }
   // Monitor parts (of the first 32) that this thread's owned cells touch. Up to
   // MREG of those that cover all of them are kept in registers: ring index of
@@ -993,7 +1013,20 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
                 if (reg == r * V + k) ev = e[r][k];
             d.out_probe[(long long)n * d.n_probes + m] = ev;
           };
-          if (probe >= 0)
+          if (flags & 512) {
+            T* const o = d.out_probe + (long long)n * d.n_probes;
+            int q = at_probe();
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              int m[V];  // a row's indices in flight together
+#pragma unroll
+              for (int k = 0; k < V; ++k)
+                if (unsigned(probe) >> (r * V + k) & 1) m[k] = entry(q++).m;
+#pragma unroll
+              for (int k = 0; k < V; ++k)
+                if (unsigned(probe) >> (r * V + k) & 1) o[m[k]] = e[r][k];
+            }
+          } else if (probe >= 0)
             record(probe, flags >> 24);
           else
             for (int q = at_probe(); q < at_end(); ++q) record(entry(q).m, entry(q).reg());
