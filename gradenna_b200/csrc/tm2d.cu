@@ -958,7 +958,7 @@ struct Layout {
   int ld = 0, rows = 0, tiles_x = 0, tiles_y = 0, n_tiles = 0, R = 32, n_gen = 0, n_int = 0;
   long long plane = 0, mon_cells = 0, n_mw = 0, n_mpts = 0;
   size_t state[2], ca, cb, psi[2], zero_end, tile_list, off[5], pts[5], mons, mw_off, mw, mring,
-      step, eacc, tasks, mpts, xch, err, blob, pv, total;
+      step, eacc, tasks, mpts, xch, err, blob, hdr, pv, total;
   size_t blob_bytes = 0;
 };
 
@@ -1101,6 +1101,21 @@ static res::Rect rect_at(const Region& g, int r, int q) {
   return res::Rect{i0, j0, std::min(g.ph, g.i0 + g.h - i0), std::min(g.pw, g.j0 + g.w - j0), g.gen};
 }
 
+// The rectangle of a cell; points mostly come in runs of one rectangle's cells.
+struct Owner {
+  const Plan& pl;
+  res::Rect x{0, 0, 0, 0, 0};
+  int idx = -1;
+  int of(int i, int j) {
+    if (i < x.i0 || i >= x.i0 + x.h || j < x.j0 || j >= x.j0 + x.w)
+      rects_of(pl, i, i + 1, j, j + 1, [&](const Region& g, int r, int q, int at) {
+        x = rect_at(g, r, q);
+        idx = at;
+      });
+    return idx;
+  }
+};
+
 // Whether a rectangle holds so many probes that reading them off sets its pace:
 // its 512 threads store them one by one, and all others wait. Only the large
 // rectangles of float kinds D and E hold that many. Time loops of 400 steps at
@@ -1111,12 +1126,32 @@ static res::Rect rect_at(const Region& g, int r, int q) {
 constexpr int kCrowd = 4096;
 static bool crowded(const Plan& pl, const GdnTmParams* p, const GdnTmPoints* pts) {
   if (p->n_probes <= kCrowd || !pts || !pts->probe_i || !pts->probe_j) return false;
-  std::vector<int> n(size_t(pl.n_rects), 0);
+  bool may = false;
+  for (const Region& g : pl.regions) may = may || g.ph * g.pw > kCrowd;
+  if (!may && p->n_probes <= p->nx * p->ny) return false;  // unless cells are named again and again
+  // A rectangle of these kinds lies in three by three bins of 64 x 64 cells.
+  const int bx = p->nx / 64 + 3, by = p->ny / 64 + 3;
+  std::vector<int> bin(size_t(bx) * by, 0);
   for (int m = 0; m < p->n_probes; ++m) {
     const int i = pts->probe_i[m], j = pts->probe_j[m];
-    rects_of(pl, i, i + 1, j, j + 1, [&](const Region&, int, int, int idx) { ++n[size_t(idx)]; });
+    if (i < 0 || i >= p->nx || j < 0 || j >= p->ny) return false;  // refused later
+    ++bin[size_t(i / 64 + 1) * by + j / 64 + 1];
   }
-  return *std::max_element(n.begin(), n.end()) > kCrowd;
+  int most = 0;
+  for (int i = 1; i < bx - 1; ++i)
+    for (int j = 1; j < by - 1; ++j) {
+      int sum = 0;
+      for (int q = 0; q < 9; ++q) sum += bin[size_t(i + q / 3 - 1) * by + j + q % 3 - 1];
+      most = std::max(most, sum);
+    }
+  if (most <= kCrowd) return false;
+  std::vector<int> n(size_t(pl.n_rects), 0);
+  Owner own{pl};
+  for (int m = 0; m < p->n_probes; ++m) {
+    const int i = pts->probe_i[m], j = pts->probe_j[m];
+    if (++n[size_t(own.of(i, j))] > kCrowd) return true;
+  }
+  return false;
 }
 
 // Bound on the copies of points in rectangles and their halos.
@@ -1213,13 +1248,15 @@ static Layout make_layout(const GdnTmParams* p, const GdnTmPoints* pts, size_t e
     // One blob, uploaded in one copy: descriptors, monitors, per-tile lists.
     const size_t nr = size_t(L.plan.n_rects);
     const size_t hdrs = std::min<size_t>(nr, res_copies(L.plan, p));
+    const size_t nt = size_t(kind_shape(esize, L.kind, false).nt);
     L.blob_bytes = sizeof(res::RDev<double>) + nr * sizeof(res::RTile) +
                    size_t(std::max(p->n_monitors, 3)) * sizeof(MonD) + 2 * (nr + 1) * sizeof(int) +
                    size_t(L.n_mw) * sizeof(MonW) +
-                   hdrs * size_t(kind_shape(esize, L.kind, false).nt) * sizeof(res::RHdr) +
+                   std::min(hdrs * nt, res_copies(L.plan, p)) * (sizeof(res::RHdr) + sizeof(int)) +
                    (hdrs + 1) * sizeof(int) +
                    res_copies(L.plan, p) * (sizeof(res::RPt) + sizeof(int)) + 16 * 16;
     L.blob = cv.take<char>(L.blob_bytes);
+    L.hdr = cv.take<res::RHdr>(hdrs * nt);
     L.pv = cv.take<char>(std::max<size_t>(size_t(L.seg) * size_t(injections(p)), 1) * esize);
     L.mring = cv.take<char>(std::max<size_t>(size_t(L.mon_cells) * L.seg, 1) * esize);
     L.eacc = cv.take<double>(1);
@@ -2030,12 +2067,17 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
     int type, m, i, j, own;
   };
   std::vector<std::vector<Copy>> in(nr);
+  Owner owner{pl};
   bool any = false;
   size_t most = 0;  // injections of a rectangle
   for (int k = 0; k < 5; ++k)
     for (int m = 0; m < counts[k]; ++m) {
-      const int i = is[k][m], j = js[k][m], halo = k < 4 ? res::TB : 0;
+      const int i = is[k][m], j = js[k][m], halo = res::TB;
       any = true;
+      if (k == 4) {
+        in[owner.of(i, j)].push_back(Copy{k, m, i, j, 1});
+        continue;
+      }
       rects_of(pl, i - halo, i + halo + 1, j - halo, j + halo + 1, [&](const Region& g, int r, int q, int idx) {
         const res::Rect x = rect_at(g, r, q);
         const int own = i >= x.i0 && i < x.i0 + x.h && j >= x.j0 && j < x.j0 + x.w;
@@ -2045,34 +2087,58 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   for (const auto& v : in)
     most = std::max(most, size_t(std::count_if(v.begin(), v.end(), [](const Copy& q) { return q.type < 4; })));
   const int staged = int(std::min(most, (kResSmem - pl.smem) / (res::TB * sizeof(T))));
-  std::vector<res::RHdr> hdr;
+  std::vector<res::RHdr> hdr;  // of threads that have entries, and their places
+  std::vector<int> hdr_at;
+  int slots = 0;
   std::vector<int> vl_off(nr + 1, 0), vl, pts_off(1, 0);
   std::vector<res::RPt> ents;
   if (any) {
     const ShapeInfo main = kind_shape(sizeof(T), L.kind, false);
-    std::vector<int> cnt(size_t(main.nt) * 4);
-    int slots = 0;
+    // Thread and register of a cell: those of its row plus those of its column.
+    struct Place {
+      std::vector<int> row_th, row_reg, col_th, col_reg;
+    } places[2];
+    for (int gen = 0; gen < 2; ++gen) {
+      const ShapeInfo s = kind_shape(sizeof(T), L.kind, gen != 0);
+      const int V = s.ew / 32, RR = s.eh / (s.nt / 32);
+      for (int r = 0; r < s.eh; ++r) {
+        places[gen].row_th.push_back(r / RR * 32);
+        places[gen].row_reg.push_back(r % RR * V);
+      }
+      for (int c = 0; c < s.ew; ++c) {
+        places[gen].col_th.push_back(c / V);
+        places[gen].col_reg.push_back(c % V);
+      }
+    }
+    std::vector<int> cnt(size_t(main.nt) * 4, 0), busy;  // busy: threads that have entries
     for (int t = 0; t < nr; ++t) {
       if (!in[t].empty()) {
         res::RTile& x = tiles[t];
         x.slot = slots++;
         const ShapeInfo s = kind_shape(sizeof(T), L.kind, x.gen != 0);
-        const int V = s.ew / 32, RR = s.eh / (s.nt / 32);
+        const Place& pc = places[x.gen != 0];
         auto place = [&](const Copy& q, int* reg) {
           const int r = q.i - x.i0 + res::TB, c = q.j - x.j0 + res::TB;
-          *reg = r % RR * V + c % V;
-          return r / RR * 32 + c / V;
+          *reg = pc.row_reg[size_t(r)] + pc.col_reg[size_t(c)];
+          return pc.row_th[size_t(r)] + pc.col_th[size_t(c)];
         };
         // Classes per thread: 0 Mx/My, 1 Jz, 2 ports, 3 probes.
         const int cls_of[5] = {2, 1, 0, 0, 3};
-        std::fill(cnt.begin(), cnt.end(), 0);
+        busy.clear();
         int reg;
-        for (const Copy& q : in[t]) ++cnt[size_t(place(q, &reg)) * 4 + cls_of[q.type]];
+        for (const Copy& q : in[t]) {
+          const int th = place(q, &reg);
+          int* const n = &cnt[size_t(th) * 4];
+          if (!(n[0] | n[1] | n[2] | n[3])) busy.push_back(th);
+          ++n[cls_of[q.type]];
+        }
+        std::sort(busy.begin(), busy.end());
         const int e0 = int(ents.size());
         int at = e0;
         ents.resize(ents.size() + in[t].size());
-        for (int th = 0; th < s.nt; ++th) {
+        for (const int th : busy) {
           int* const n = &cnt[size_t(th) * 4];
+          hdr_at.push_back(x.slot * s.nt + th);
           hdr.push_back(res::RHdr{at - e0, unsigned(n[0]) | unsigned(n[1]) << 16,
                                   unsigned(n[2]) | unsigned(n[3]) << 16, 0, 0, 0, 0, 0, 0});
           for (int k = 0; k < 4; ++k) {
@@ -2103,9 +2169,8 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
         std::vector<std::pair<int, int>> port_val;  // (m, value)
         for (const Copy& q : in[t])
           if (q.type == 0) port_val.push_back({q.m, port++});
-        res::RHdr* const h0 = &hdr[hdr.size() - size_t(s.nt)];
-        for (int th = 0; th < s.nt; ++th) {
-          res::RHdr& h = h0[th];
+        for (size_t k = hdr.size() - busy.size(); k < hdr.size(); ++k) {
+          res::RHdr& h = hdr[k];
           res::RPt* x0 = ents.data() + e0 + h.first;
           const int n_mag = int(h.n01 & 0xffff), n_jz = int(h.n01 >> 16), n_port = int(h.n23 & 0xffff);
           for (int cls = 0; cls < 2; ++cls) {
@@ -2149,6 +2214,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
               if (pv.first == e.m) e.w |= unsigned(pv.second) << 10;
           }
         }
+        for (const int th : busy) std::fill_n(&cnt[size_t(th) * 4], 4, 0);
       }
       vl_off[t + 1] = int(vl.size());
       if (!in[t].empty()) pts_off.push_back(int(ents.size()));
@@ -2165,7 +2231,8 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   d.mw = reinterpret_cast<const MonW*>(dev(append(blob, mw.data(), mw.size())));
   rd.vl_off = nullptr;
   if (any) rd.vl_off = reinterpret_cast<const int*>(dev(append(blob, vl_off.data(), vl_off.size())));
-  rd.hdr = reinterpret_cast<const res::RHdr*>(dev(append(blob, hdr.data(), hdr.size())));
+  rd.hdr = reinterpret_cast<const res::RHdr*>(ws + L.hdr);
+  const size_t a_hdr = append(blob, hdr.data(), hdr.size()), a_at = append(blob, hdr_at.data(), hdr_at.size());
   rd.pts_off = reinterpret_cast<const int*>(dev(append(blob, pts_off.data(), pts_off.size())));
   rd.pts = reinterpret_cast<const res::RPt*>(dev(append(blob, ents.data(), ents.size())));
   rd.vl = reinterpret_cast<const int*>(dev(append(blob, vl.data(), vl.size())));
@@ -2181,6 +2248,15 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
     GDN_BAD_ARG("internal: %zu bytes of tables, layout sized for %zu", blob.size(), L.blob_bytes);
   // Pageable: staged when the call returns, so the image may go away.
   GDN_TRY_CUDA(cudaMemcpyAsync(base, blob.data(), blob.size(), cudaMemcpyHostToDevice, stream));
+  // Few threads have entries: their headers go to their places here.
+  if (!hdr.empty()) {
+    GDN_TRY_CUDA(cudaMemsetAsync(ws + L.hdr, 0, size_t(slots) * kind_shape(sizeof(T), L.kind, false).nt *
+                                                    sizeof(res::RHdr), stream));
+    res::tm_headers<<<unsigned(div_up((long long)hdr.size(), 256)), 256, 0, stream>>>(
+        reinterpret_cast<const res::RHdr*>(dev(a_hdr)), reinterpret_cast<const int*>(dev(a_at)),
+        int(hdr.size()), reinterpret_cast<res::RHdr*>(ws + L.hdr));
+    count_launches(1);
+  }
   R.d_rd = reinterpret_cast<const res::RDev<T>*>(base + a_rd);
   R.d_rtiles = reinterpret_cast<const res::RTile*>(base + a_tiles);
   R.err = reinterpret_cast<int*>(ws + L.err);

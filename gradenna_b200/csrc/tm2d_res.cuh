@@ -1124,6 +1124,14 @@ __global__ void __launch_bounds__(S::NT, 1) tm_res(RArgs<typename S::T> a) {
     body<S, false>(D, tl, a, U);
 }
 
+// Headers to their places among all threads' (zeroed beforehand). Uploaded for
+// every thread, 16 KB a rectangle that holds points, they were most of what a run
+// of a few steps with scattered points took.
+__global__ void tm_headers(const RHdr* in, const int* at, int n, RHdr* out) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < n) out[at[q]] = in[q];
+}
+
 // Injected values of steps [seg0, seg0 + cnt): one thread per injection and
 // FOLD steps (blockIdx.y), problem blockIdx.z. The products are formed like
 // the tile kernels' (src_term, mx_term, my_term and the port term).
