@@ -2006,7 +2006,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
       for (int q = 0; q < g.nc; ++q) {
         const res::Rect x = rect_at(g, r, q);
         const int idx = g.first + r * g.nc + q;
-        tiles[idx] = res::RTile{0, idx, -1, x.i0, x.j0, x.h, x.w, x.gen};
+        tiles[idx] = res::RTile{idx, -1, x.i0, x.j0, x.h, x.w, x.gen};
       }
 
   // Monitors and their parts per rectangle.
@@ -2239,7 +2239,6 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   rd.xch = reinterpret_cast<uint4*>(ws + L.xch);
   rd.pv = reinterpret_cast<const T*>(ws + L.pv);
   rd.n_inj = int(injections(p));
-  rd.dft_f64 = p->dft_f64 != 0;
   rd.val_at = int(pl.smem / sizeof(T));
   rd.val_cap = staged;
   rd.d = d;
@@ -2262,31 +2261,6 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   R.err = reinterpret_cast<int*>(ws + L.err);
   return GDN_OK;
 }
-
-// Problems advanced together by resident launches (a single run: one).
-template <typename T>
-struct Wave {
-  const res::RDev<T>* devs = nullptr;
-  const res::RTile* tiles = nullptr;
-  int* err = nullptr;
-  int n_prob = 0, n_tiles = 0, kind = 0, seg = 0, n_steps = 0, kmax = 0;
-  long long inj_max = 0, mon_max = 0;
-  bool f32 = false, f64 = false;  // DFT accumulator types present
-  size_t smem = 0;
-
-  void add(const GdnTmParams* p, const Run<T>& R) {
-    ++n_prob;
-    n_tiles += int(R.rtiles.size());
-    n_steps = std::max(n_steps, p->n_steps);
-    kmax = std::max(kmax, p->n_freq);
-    inj_max = std::max(inj_max, injections(p));
-    smem = std::max(smem, R.rsmem);
-    if (!R.mons.empty()) {
-      mon_max = std::max(mon_max, R.L.mon_cells);
-      (p->dft_f64 ? f64 : f32) = true;
-    }
-  }
-};
 
 // One cooperative launch. Tiles of two such launches wait only for their own,
 // but each needs all of its tiles on the device: launches of this process on
@@ -2319,15 +2293,16 @@ static int launch_coop(const res::RArgs<typename S::T>& a, int n_tiles, size_t s
 }
 
 template <typename T, typename A>
-static void launch_seg_fold(const Wave<T>& w, const Dev<T>& d, int seg0, cudaStream_t s) {
-  const size_t sm = size_t(4) * res::FOLD * w.kmax * sizeof(A);
+static void launch_seg_fold(const Run<T>& R, int seg0, cudaStream_t s) {
+  const int K = R.d.n_freq;
+  const size_t sm = size_t(4) * res::FOLD * K * sizeof(A);
   auto launch = [&](auto km) {
     constexpr int KM = decltype(km)::value, NT = res::fold_threads<T, A>(KM);
-    res::tm_seg_fold<T, A, KM><<<unsigned(div_up(w.mon_max, NT)), NT, sm, s>>>(d, seg0, w.seg);
+    res::tm_seg_fold<T, A, KM><<<unsigned(div_up(R.L.mon_cells, NT)), NT, sm, s>>>(R.d, seg0, R.L.seg);
   };
-  if (w.kmax <= 4)
+  if (K <= 4)
     launch(std::integral_constant<int, 4>{});
-  else if (w.kmax <= 8)
+  else if (K <= 8)
     launch(std::integral_constant<int, 8>{});
   else
     launch(std::integral_constant<int, KMAX>{});
@@ -2338,32 +2313,37 @@ static void launch_seg_fold(const Wave<T>& w, const Dev<T>& d, int seg0, cudaStr
 static thread_local int t_hold = -1;
 constexpr int kHoldPolls = 1 << 12;  // then a few milliseconds of polls
 
-// All time steps of a wave: per segment the value table, the tiles (one
-// cooperative launch when they all fit, else one launch per block) and the
-// DFT sums.
+// All time steps of a run: per segment the value table, the rectangles (one
+// cooperative launch) and the DFT sums.
 template <typename T>
-static int run_wave(const Wave<T>& w, const Dev<T>& d, cudaStream_t stream) {
-  return with_kind<T>(w.kind, [&](auto sh, auto sh2) -> int {
+static int run_segments(const GdnTmParams* p, const Run<T>& R, cudaStream_t stream) {
+  return with_kind<T>(R.L.kind, [&](auto sh, auto sh2) -> int {
     using S = decltype(sh);
     using S2 = decltype(sh2);
+    const long long inj = injections(p);
+    const int n_rects = int(R.rtiles.size()), seg = R.L.seg;
     int st;
     GDN_TRY_CUDA(cudaFuncSetAttribute(res::tm_res<S, S2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(kResSmem)));
     uint64_t k = 0;
-    for (int seg0 = 0; seg0 < w.n_steps; seg0 += w.seg) {
-      const int cnt = std::min(w.seg, w.n_steps - seg0);
-      if (w.inj_max > 0) {
-        res::tm_values<T><<<dim3(unsigned(div_up(w.inj_max, 128)), unsigned(div_up(cnt, res::FOLD)),
-                                 unsigned(w.n_prob)), 128, 0, stream>>>(w.devs, seg0, w.seg);
+    for (int seg0 = 0; seg0 < p->n_steps; seg0 += seg) {
+      const int cnt = std::min(seg, p->n_steps - seg0);
+      if (inj > 0) {
+        res::tm_values<T><<<dim3(unsigned(div_up(inj, 128)), unsigned(div_up(cnt, res::FOLD))), 128, 0,
+                            stream>>>(R.d_rd, seg0, seg);
         ++k;
       }
       const int b0 = seg0 / res::TB, b1 = int(div_up(seg0 + cnt, res::TB));
-      res::RArgs<T> a{w.devs, w.tiles, w.err, b0, b1, seg0, t_hold < 0 ? res::POLLS : kHoldPolls, t_hold};
-      if ((st = launch_coop<S, S2>(a, w.n_tiles, w.smem, stream))) return st;
+      res::RArgs<T> a{R.d_rd, R.d_rtiles, R.err, b0, b1, seg0, t_hold < 0 ? res::POLLS : kHoldPolls, t_hold};
+      if ((st = launch_coop<S, S2>(a, n_rects, R.rsmem, stream))) return st;
       ++k;
-      if (w.f64) launch_seg_fold<T, double>(w, d, seg0, stream);
-      if (w.f32) launch_seg_fold<T, float>(w, d, seg0, stream);
-      k += int(w.f64) + int(w.f32);
+      if (!R.mons.empty()) {
+        if (p->dft_f64)
+          launch_seg_fold<T, double>(R, seg0, stream);
+        else
+          launch_seg_fold<T, float>(R, seg0, stream);
+        ++k;
+      }
     }
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) {
@@ -2430,15 +2410,8 @@ static int run(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTmBuffers*
   } guard{ws, own, stream};
   if ((st = prepare(p, pts, b, ws, R, stream))) return st;
   if (R.L.res) {
-    Wave<T> w;
-    w.add(p, R);
-    w.devs = R.d_rd;
-    w.tiles = R.d_rtiles;
-    w.err = R.err;
-    w.kind = R.L.kind;
-    w.seg = R.L.seg;
     LoopTimer timer(stream, double(p->nx) * p->ny * p->n_steps, div_up(p->n_steps, res::TB));
-    st = run_wave(w, R.d, stream);
+    st = run_segments(p, R, stream);
     timer.stop(st == GDN_OK);
     return st ? st : finalize(p, b, R, stream);
   }

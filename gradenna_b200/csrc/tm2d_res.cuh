@@ -76,13 +76,13 @@ struct __align__(16) RHdr {
 };
 constexpr int MAXE = 512;  // entries of a rectangle staged in shared memory
 
-// Everything a rectangle needs besides Dev: one per problem.
+// Everything a rectangle needs besides Dev: one per run.
 template <typename T>
 struct RDev {
   Dev<T> d;
   uint4* xch;          // words in flight: [parity][NF + 2 NP][padded plane]
   const T* pv;         // [step - seg0][n_inj] injected values
-  int n_inj, dft_f64;
+  int n_inj;
   // A rectangle's first val_cap injections are staged in shared memory, from
   // element val_at on. As many as the largest rectangle holds wherever they fit:
   // fetched from pv entry by entry instead, past a fixed 256 of them, the 360 of
@@ -96,14 +96,14 @@ struct RDev {
   const RPt* pts;
 };
 
-// A CTA of a launch: problem, rectangle and its index, header slot or -1.
+// A CTA of a launch: a rectangle and its index, header slot or -1.
 struct RTile {
-  int prob, idx, slot, i0, j0, h, w, gen;
+  int idx, slot, i0, j0, h, w, gen;
 };
 
 template <typename T>
 struct RArgs {
-  const RDev<T>* devs;
+  const RDev<T>* dev;
   const RTile* tiles;
   int* err;
   int blk0, blk1, seg0;  // blocks [blk0, blk1); ring and value slot 0 is step seg0
@@ -1113,7 +1113,7 @@ __global__ void __launch_bounds__(S::NT, 1) tm_res(RArgs<typename S::T> a) {
   const RTile tl = a.tiles[blockIdx.x];
   // A rectangle of an earlier segment (or of this one) gave up: nothing to do.
   if (__syncthreads_or(*reinterpret_cast<const volatile int*>(a.err))) return;
-  const int* src = reinterpret_cast<const int*>(a.devs + tl.prob);
+  const int* src = reinterpret_cast<const int*>(a.dev);
   for (int q = threadIdx.x; q < int(sizeof(RDev<T>) / sizeof(int)); q += S::NT)
     reinterpret_cast<int*>(sdev)[q] = src[q];
   __syncthreads();
@@ -1133,11 +1133,11 @@ __global__ void tm_headers(const RHdr* in, const int* at, int n, RHdr* out) {
 }
 
 // Injected values of steps [seg0, seg0 + cnt): one thread per injection and
-// FOLD steps (blockIdx.y), problem blockIdx.z. The products are formed like
+// FOLD steps (blockIdx.y). The products are formed like
 // the tile kernels' (src_term, mx_term, my_term and the port term).
 template <typename T>
-__global__ void __launch_bounds__(128) tm_values(const RDev<T>* devs, int seg0, int seg) {
-  const RDev<T>& D = devs[blockIdx.z];
+__global__ void __launch_bounds__(128) tm_values(const RDev<T>* dev, int seg0, int seg) {
+  const RDev<T>& D = *dev;
   const Dev<T>& d = D.d;
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= D.n_inj) return;
