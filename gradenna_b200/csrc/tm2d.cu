@@ -931,8 +931,10 @@ static Plan make_plan(const GdnTmParams* p, size_t esize, const Cfg& c, int kind
 // wait for one another: with more of them than SMs the state would have to go
 // through memory every block. Tried with one launch a block, 1024 x 1024 f64
 // took 36 ms for 1000 steps where the tile kernels take 30. Batches keep the
-// tile kernels too: they fill the chip already (24 problems of 128^2 to 512^2,
-// gradients: 0.45 s; 0.49 s with resident launches one after another).
+// tile kernels: one resident launch a problem, one after another, gave nothing
+// (24 problems of 128^2 to 512^2, gradients, whole calls with the library's
+// allocation of their scratch: 0.49 s against 0.45 s); several problems in one
+// launch were not tried.
 static int choose_kind(const GdnTmParams* p, size_t esize, const Cfg& c, Plan* out) {
   const int sms = sm_count();
   for (int k = 0; k < kinds(esize); ++k) {
@@ -1168,9 +1170,12 @@ static long long injections(const GdnTmParams* p) {
   return (long long)p->n_sources + p->n_mx + p->n_my + p->n_ports;
 }
 
-// Steps per segment: the ring within 256 MiB, the value table within 64 MiB.
-// Between segments the state goes through memory once (about 15 us at 1024^2
-// against 6 us a block), so a few hundred steps make that small.
+// Steps per segment: the ring within 256 MiB, the value table within 64 MiB, but
+// never fewer than FOLD, so that a full grid's ring can take more (12 B a cell
+// and step in float: 400 MB at 1024^2, 2 GiB at most, use_res). Between segments
+// the state goes through memory once (about 15 us at 1024^2 against 6 us a
+// step): small against a few hundred steps, 8 % of the FOLD steps that a
+// full-grid ring leaves, whose own stores and sums cost more.
 static int seg_steps(int n_steps, long long mon, long long inj, size_t esize) {
   long long s = std::min<long long>(res::SEG_MAX, div_up(std::max(n_steps, 1), res::FOLD) * res::FOLD);
   if (mon > 0) s = std::min<long long>(s, (256LL << 20) / (mon * (long long)esize));

@@ -28,16 +28,17 @@
 //     partial sums as tm_dft_fold.
 //
 // What bounds it: not memory (the state stays in registers; only ring, frame
-// and value traffic is left) but a block's chain. At 1024 x 1024 f32 with a
-// 512 x 512 design monitor and contour currents a block of four steps takes
-// 22 us, 13.7 us without points: half steps, the row exchange and two barriers
-// a step, about 4 us for send and receive, then points and ring stores.
+// and value traffic is left: 4 MB of DRAM a block at 1024 x 1024) but a block's
+// chain. At 1024 x 1024 f32 with a 512 x 512 design monitor and contour currents a
+// block of four steps takes 21 us, 12 us with one source: half steps, the row
+// exchange and two barriers a step, about 4 us for send and receive, then points
+// and ring stores.
 // Measured on B200 against the tile kernels alone, whole calls:
 //   70 x 53 f32, 300 steps, 2 frequencies                  2.8 ms -> 1.5 ms
-//   140 x 140 f32 gradient, 2 x 3500 steps                41.9 ms -> 20.6 ms
-//   280 x 280 f64 gradient, 2 x 7000 steps                  84 ms -> 57 ms
-//   517 x 384 f32, 2000 steps, 8 frequencies, whole grid  18.3 ms -> 11.7 ms
-//   1024 x 1024 f32 gradient, 2 x 8000 steps               143 ms -> 108 ms
+//   140 x 140 f32 gradient, 2 x 3500 steps                41.9 ms -> 19.7 ms
+//   280 x 280 f64 gradient, 2 x 7000 steps                  84 ms -> 53 ms
+//   517 x 384 f32, 2000 steps, 8 frequencies, whole grid  18.3 ms -> 9.6 ms
+//   1024 x 1024 f32 gradient, 2 x 8000 steps               143 ms -> 98 ms
 #pragma once
 
 namespace res {

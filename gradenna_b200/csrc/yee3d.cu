@@ -17,9 +17,10 @@
 // lives in full padded volumes (zero outside the slabs) indexed like the
 // fields; only slab cells touch them. ca, cb are laid out like the fields when a
 // run starts, the CPML coefficients as tables by node.
-//   What bounds it: the L2 round trip of a plane's loads with 16 warps an SM
-// (ncu at 160 x 160 x 64 f32: issue 12 %, long-scoreboard stalls 70 %, H 18 us
-// and E 21 us a step; their 160 MB at L2 rates would take about 20 us a step).
+//   What bounds it: the round trip of a plane's loads to L2 with 14 warps an SM
+// (ncu at 160 x 160 x 64 f32, caches cold: issue 44 % and 39 %, half of the stalls
+// long scoreboard, L2 27 %; in a run H 16 us and E 20 us a step, waits for the
+// kernel before included).
 // Coefficients are fetched before the wait for the previous kernel (300 -> 288 ms).
 // One cell a thread, 8 x 32 boxes, was issue bound: 252 (H) and 300 (E) warp
 // instructions per 32 cells. More warps with fewer registers lose to spills (5
