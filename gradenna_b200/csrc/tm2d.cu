@@ -1166,8 +1166,10 @@ static size_t res_copies(const Plan& pl, const GdnTmParams* p) {
   return np * std::min<size_t>(k * k, size_t(pl.n_rects)) + size_t(p->n_probes);
 }
 
-static long long injections(const GdnTmParams* p) {
-  return (long long)p->n_sources + p->n_mx + p->n_my + p->n_ports;
+// Bound on the injected values of a step: a point counts in every rectangle whose
+// halo holds it.
+static long long res_values(const Plan& pl, const GdnTmParams* p) {
+  return (long long)res_copies(pl, p) - p->n_probes;
 }
 
 // Steps per segment: the ring within 256 MiB, the value table within 64 MiB, but
@@ -1176,10 +1178,10 @@ static long long injections(const GdnTmParams* p) {
 // the state goes through memory once (about 15 us at 1024^2 against 6 us a
 // step): small against a few hundred steps, 8 % of the FOLD steps that a
 // full-grid ring leaves, whose own stores and sums cost more.
-static int seg_steps(int n_steps, long long mon, long long inj, size_t esize) {
+static int seg_steps(int n_steps, long long mon, long long vals, size_t esize) {
   long long s = std::min<long long>(res::SEG_MAX, div_up(std::max(n_steps, 1), res::FOLD) * res::FOLD);
   if (mon > 0) s = std::min<long long>(s, (256LL << 20) / (mon * (long long)esize));
-  if (inj > 0) s = std::min<long long>(s, (64LL << 20) / (inj * (long long)esize));
+  if (vals > 0) s = std::min<long long>(s, (64LL << 20) / (vals * (long long)esize));
   return int(std::max<long long>(res::FOLD, s / res::FOLD * res::FOLD));
 }
 
@@ -1217,7 +1219,7 @@ static Layout make_layout(const GdnTmParams* p, const GdnTmPoints* pts, size_t e
       rects_of(L.plan, bx[1], bx[1] + bx[3], bx[2], bx[2] + bx[4],
                [&](const Region&, int, int, int) { ++L.n_mw; });
     L.mon_cells = padded_cells(p, pts);
-    L.seg = ring_steps > 0 ? ring_steps : seg_steps(p->n_steps, L.mon_cells, injections(p), esize);
+    L.seg = ring_steps > 0 ? ring_steps : seg_steps(p->n_steps, L.mon_cells, res_values(L.plan, p), esize);
     L.R = L.seg;
   } else if (ring_steps > 0) {
     L.R = ring_steps;
@@ -1262,7 +1264,7 @@ static Layout make_layout(const GdnTmParams* p, const GdnTmPoints* pts, size_t e
                    res_copies(L.plan, p) * (sizeof(res::RPt) + sizeof(int)) + 16 * 16;
     L.blob = cv.take<char>(L.blob_bytes);
     L.hdr = cv.take<res::RHdr>(hdrs * nt);
-    L.pv = cv.take<char>(std::max<size_t>(size_t(L.seg) * size_t(injections(p)), 1) * esize);
+    L.pv = cv.take<char>(std::max<size_t>(size_t(L.seg) * size_t(res_values(L.plan, p)), 1) * esize);
     L.mring = cv.take<char>(std::max<size_t>(size_t(L.mon_cells) * L.seg, 1) * esize);
     L.eacc = cv.take<double>(1);
     L.total = cv.bytes();
@@ -2098,6 +2100,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   std::vector<int> vl_off(nr + 1, 0), vl, pts_off(1, 0);
   std::vector<res::RPt> ents;
   if (any) {
+    static_assert(res::F32E::R * res::F32E::V <= 32, "a mask holds a thread's registers");
     const ShapeInfo main = kind_shape(sizeof(T), L.kind, false);
     // Thread and register of a cell: those of its row plus those of its column.
     struct Place {
@@ -2116,6 +2119,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
       }
     }
     std::vector<int> cnt(size_t(main.nt) * 4, 0), busy;  // busy: threads that have entries
+    std::vector<std::pair<int, int>> sorted;             // (layer, kind, register), injection
     for (int t = 0; t < nr; ++t) {
       if (!in[t].empty()) {
         res::RTile& x = tiles[t];
@@ -2145,7 +2149,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
           int* const n = &cnt[size_t(th) * 4];
           hdr_at.push_back(x.slot * s.nt + th);
           hdr.push_back(res::RHdr{at - e0, unsigned(n[0]) | unsigned(n[1]) << 16,
-                                  unsigned(n[2]) | unsigned(n[3]) << 16, 0, 0, 0, 0, 0, 0});
+                                  unsigned(n[2]) | unsigned(n[3]) << 16, 0, 0, 0, 0, 0});
           for (int k = 0; k < 4; ++k) {
             const int here = n[k];
             n[k] = at;
@@ -2162,7 +2166,7 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
           ents[cnt[size_t(th) * 4 + cls_of[q.type]]++] = e;
         }
         // Values: ports in port order, then every thread's magnetic and electric
-        // currents, by register where no register has two.
+        // currents by layer and register.
         int val = 0;
         for (const Copy& q : in[t])
           if (q.type == 0) {
@@ -2178,35 +2182,44 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
           res::RHdr& h = hdr[k];
           res::RPt* x0 = ents.data() + e0 + h.first;
           const int n_mag = int(h.n01 & 0xffff), n_jz = int(h.n01 >> 16), n_port = int(h.n23 & 0xffff);
+          h.v = unsigned(int(vl.size()) - v0);
+          if (int(h.v) + n_mag + n_jz > staged) h.how |= 1;
           for (int cls = 0; cls < 2; ++cls) {
             res::RPt* const a = cls == 0 ? x0 : x0 + n_mag;
             const int n = cls == 0 ? n_mag : n_jz;
+            // Layers: an entry's is the number of earlier ones of its cell.
             unsigned mask[2] = {0, 0};
-            bool once = n > 0;
+            bool once = true;
             for (int q = 0; q < n; ++q) {
               unsigned& mk = mask[cls == 0 ? a[q].kind() : 0];
-              once = once && a[q].reg() < 32 && !(mk >> a[q].reg() & 1);
-              if (a[q].reg() < 32) mk |= 1u << a[q].reg();
+              once = once && !(mk >> a[q].reg() & 1);
+              mk |= 1u << a[q].reg();
             }
-            if (once)
-              std::sort(a, a + n, [](const res::RPt& x, const res::RPt& y) {
-                return std::make_pair(x.kind(), x.reg()) < std::make_pair(y.kind(), y.reg());
-              });
-            const int first = int(vl.size()) - v0;
-            for (int q = 0; q < n; ++q) {
-              a[q].w |= unsigned(int(vl.size()) - v0) << 10;
-              vl.push_back(a[q].m);
-            }
-            if (once && first + n <= staged) {
-              h.dense |= 1u << cls;
-              if (cls == 0) {
-                h.m_hx = mask[0];
-                h.m_hy = mask[1];
-                h.v_h = static_cast<unsigned short>(first);
-              } else {
-                h.m_e = mask[0];
-                h.v_e = static_cast<unsigned short>(first);
+            if (once) {
+              std::sort(a, a + n, [](const res::RPt& x, const res::RPt& y) { return x.w < y.w; });
+              for (int q = 0; q < n; ++q) vl.push_back(a[q].m);
+            } else {
+              int seen[64] = {};
+              sorted.clear();
+              for (int q = 0; q < n; ++q) {
+                const int at_reg = (cls == 0 ? a[q].kind() : 0) * 32 + a[q].reg();
+                sorted.push_back({seen[at_reg]++ * 64 + at_reg, a[q].m});
               }
+              std::sort(sorted.begin(), sorted.end());
+              std::fill_n(a, n, res::RPt{0, 0});
+              for (const auto& [key, m] : sorted) {
+                vl.push_back(m);
+                if (key < 64) continue;
+                res::RPt& layer = a[key / 64 - 1];
+                (key & 32 ? layer.w : reinterpret_cast<unsigned&>(layer.m)) |= 1u << (key & 31);
+              }
+              h.how |= cls == 0 ? 2 : 8;
+            }
+            if (cls == 0) {
+              h.m_hx = mask[0];
+              h.m_hy = mask[1];
+            } else {
+              h.m_e = mask[0];
             }
           }
           // Probes by register (a kernel reads them off in that order where no
@@ -2243,7 +2256,9 @@ static int prepare_res(const GdnTmParams* p, const GdnTmPoints* pts, const GdnTm
   rd.vl = reinterpret_cast<const int*>(dev(append(blob, vl.data(), vl.size())));
   rd.xch = reinterpret_cast<uint4*>(ws + L.xch);
   rd.pv = reinterpret_cast<const T*>(ws + L.pv);
-  rd.n_inj = int(injections(p));
+  rd.n_vals = int(vl.size());
+  if ((long long)vl.size() > res_values(pl, p))
+    GDN_BAD_ARG("internal: %zu injected values, layout sized for %lld", vl.size(), res_values(pl, p));
   rd.val_at = int(pl.smem / sizeof(T));
   rd.val_cap = staged;
   rd.d = d;
@@ -2325,7 +2340,7 @@ static int run_segments(const GdnTmParams* p, const Run<T>& R, cudaStream_t stre
   return with_kind<T>(R.L.kind, [&](auto sh, auto sh2) -> int {
     using S = decltype(sh);
     using S2 = decltype(sh2);
-    const long long inj = injections(p);
+    const int vals = R.rd.n_vals;
     const int n_rects = int(R.rtiles.size()), seg = R.L.seg;
     int st;
     GDN_TRY_CUDA(cudaFuncSetAttribute(res::tm_res<S, S2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2333,8 +2348,8 @@ static int run_segments(const GdnTmParams* p, const Run<T>& R, cudaStream_t stre
     uint64_t k = 0;
     for (int seg0 = 0; seg0 < p->n_steps; seg0 += seg) {
       const int cnt = std::min(seg, p->n_steps - seg0);
-      if (inj > 0) {
-        res::tm_values<T><<<dim3(unsigned(div_up(inj, 128)), unsigned(div_up(cnt, res::FOLD))), 128, 0,
+      if (vals > 0) {
+        res::tm_values<T><<<dim3(unsigned(div_up(vals, 128)), unsigned(div_up(cnt, res::FOLD))), 128, 0,
                             stream>>>(R.d_rd, seg0, seg);
         ++k;
       }

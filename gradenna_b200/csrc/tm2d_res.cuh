@@ -53,10 +53,9 @@ struct Rect {
   int i0, j0, h, w, gen;
 };
 
-// A point copy in the thread that holds its cell: `m` its own index; w packs
-// register r * V + k (8 bits), kind (2 bits: 0 Hx, 1 Hy for magnetic currents; 1
-// = owner for ports) and the index of its value among the rectangle's
-// injections (22 bits; a port's is also its number in the rectangle).
+// A port or probe copy in the thread that holds its cell: `m` its own index; w
+// packs register r * V + k (8 bits), kind (2 bits: 1 = owner for ports) and a
+// port's number in the rectangle (22 bits), which is also that of its value.
 struct __align__(8) RPt {
   int m;
   unsigned w;
@@ -65,15 +64,21 @@ struct __align__(8) RPt {
   __host__ __device__ int val() const { return int(w >> 10); }
 };
 // A thread's entries of its rectangle: first, then the counts of Mx/My, Jz,
-// ports and probes (16 bits each). Where no cell of the thread has two magnetic
-// (two electric) current entries and their values are staged, `dense` bit 0
-// (1) is set, masks hold the cells' registers, and the values follow one
-// another in the order of the bits from v_h (Hx, then Hy) and v_e.
+// ports and probes (16 bits each). Currents are added by masks of the registers
+// whose cells have one: the values follow one another from index v of the
+// rectangle's on, Hx then Hy by register, then Jz (from v plus the count of
+// Mx/My). Cells with several currents have the second ones in another layer of
+// masks, and so on: `how` bit 1 (3) says that magnetic (electric) layers follow as
+// {Hx mask, Hy mask} ({Ez mask, 0}) in the class's entries up to a pair of zeros;
+// bit 0 that the values are not staged. us for 160 steps at 1024 x 1024 f32, an
+// entry at a time, each value through an index -> by layers, values in order,
+// staged by asynchronous copies (tile kernels): 150 x 150 Jz 4209 -> 833 (1926),
+// 16 x 16 Jz named twice 3246 -> 576 (989). A row's values loaded together first
+// spilled (F32E: 72 -> 440 bytes) and cost the 1024 x 1024 gradient an eighth.
 struct __align__(16) RHdr {
   int first;
-  unsigned n01, n23, dense;
-  unsigned m_hx, m_hy, m_e;
-  unsigned short v_h, v_e;
+  unsigned n01, n23, how;
+  unsigned m_hx, m_hy, m_e, v;
 };
 constexpr int MAXE = 512;  // entries of a rectangle staged in shared memory
 
@@ -82,16 +87,16 @@ template <typename T>
 struct RDev {
   Dev<T> d;
   uint4* xch;          // words in flight: [parity][NF + 2 NP][padded plane]
-  const T* pv;         // [step - seg0][n_inj] injected values
-  int n_inj;
+  const T* pv;         // [step - seg0][n_vals] injected values, by rectangle
+  int n_vals;
   // A rectangle's first val_cap injections are staged in shared memory, from
   // element val_at on. As many as the largest rectangle holds wherever they fit:
   // fetched from pv entry by entry instead, past a fixed 256 of them, the 360 of
   // a rectangle that a flux contour crosses set the pace of the whole 1024 x 1024
   // adjoint run (38.1 us a block of four steps; staged 17.8).
   int val_at, val_cap;
-  const int* vl_off;   // per rectangle CSR over vl: injections it holds
-  const int* vl;       // injection index (Jz, Mx, My, ports)
+  const int* vl_off;   // per rectangle CSR over vl: its values
+  const int* vl;       // their injection (Jz, Mx, My, ports)
   const RHdr* hdr;     // [slot][NT]
   const int* pts_off;  // [slot] CSR over pts
   const RPt* pts;
@@ -248,6 +253,13 @@ __device__ __forceinline__ unsigned get_pair(const uint4* p, int, float& u, floa
 __device__ __forceinline__ unsigned get_pair(const uint4* p, int n, double& u, double& v, unsigned blk) {
   return get_one(p, u, blk) | get_one(p + n, v, blk);
 }
+// One value from memory to shared memory, not waited for.
+template <typename T>
+__device__ __forceinline__ void copy_async(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(unsigned(__cvta_generic_to_shared(dst))),
+               "l"(src), "n"(int(sizeof(T)))
+               : "memory");
+}
 // V adjacent values between registers and memory: for V of 2 and 4 one access
 // (the address is a multiple of V values).
 template <typename T, int V>
@@ -398,7 +410,8 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
     return owned(r, k) && ((rows >> (16 + r) | cols >> (16 + k)) & 1);
   };
   // Flags: 1 Mx/My, 2 Jz, 4 ports, 8 probes, 16 monitors, 32 a port in the warp,
-  // 64 a y slab in the warp, 128 (256) magnetic (electric) entries dense.
+  // 64 a y slab in the warp, 128 values not staged, 256 (1024) more magnetic
+  // (electric) layers.
   unsigned flags = 0;
   int hd_first = 0;
   unsigned n01 = 0, n23 = 0;
@@ -408,7 +421,7 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
     n01 = hd.n01;
     n23 = hd.n23;
     flags |= (n01 & 0xffff ? 1u : 0u) | (n01 >> 16 ? 2u : 0u) | (n23 & 0xffff ? 4u : 0u) |
-             (n23 >> 16 ? 8u : 0u) | hd.dense << 7;
+             (n23 >> 16 ? 8u : 0u) | hd.how << 7;
   }
   // Entry q of this thread's list; begin and end of a class in it.
   auto entry = [&](int q) {
@@ -743,13 +756,10 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
   const T dt_mu = d.dt_mu, inv_dx = d.inv_dx, inv_dy = d.inv_dy;
 #pragma unroll 1
   for (int b = a.blk0; b < min(a.blk1, (d.n_steps + TB - 1) / TB); ++b) {
-    // Injected values of the block: [sub-step][injection].
-    {
-      const int nvs = U.nvs, nsub = min(TB, d.n_steps - b * TB);
-      for (int q = threadIdx.x; q < nvs * nsub; q += S::NT) {
-        const int s = q / nvs, v = q - s * nvs;
-        sm[D.val_at + q] = D.pv[(long long)(b * TB + s - a.seg0) * D.n_inj + D.vl[U.vb + v]];
-      }
+    // Injected values of the block, [sub-step][value], while the halo comes.
+    for (int s = 0; s < min(TB, d.n_steps - b * TB); ++s) {
+      const T* const src = D.pv + (long long)(b * TB + s - a.seg0) * D.n_vals + U.vb;
+      for (int q = threadIdx.x; q < U.nvs; q += S::NT) copy_async(sm + D.val_at + s * U.nvs + q, src + q);
     }
     if (b == a.blk0) {
       load(b & 1);
@@ -759,6 +769,7 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
       unpack();
     }
     publish_e();
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (U.fail) {
       if (threadIdx.x == 0) atomicExch(a.err, 1);
@@ -826,40 +837,41 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
           }
         }
       }
-      // Value of injection `v` of the rectangle at this step.
-      auto value = [&](int v) {
-        return v < U.nvs ? sm[D.val_at + (n - b * TB) * U.nvs + v]
-                         : D.pv[(long long)(n - a.seg0) * D.n_inj + D.vl[U.vb + v]];
-      };
+      // The rectangle's values of this step, staged or in memory.
       const T* const staged = sm + D.val_at + (n - b * TB) * U.nvs;
-      if ((flags & 129) == 129) {  // Mx / My, one a cell at most
-        const RHdr& hd = D.hdr[(long long)tl.slot * S::NT + threadIdx.x];
-        const T* v = staged + hd.v_h;
-        const unsigned mx = hd.m_hx, my = hd.m_hy;
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int k = 0; k < V; ++k)
-            if (mx >> (r * V + k) & 1) hx[r][k] += -*v++;
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int k = 0; k < V; ++k)
-            if (my >> (r * V + k) & 1) hy[r][k] += -*v++;
-      } else if (flags & 1) {
-        for (int q = hd_first; q < at_jz(); ++q) {
-          const RPt p = entry(q);
-          const T v = value(p.val());
+      auto in_memory = [&]() { return D.pv + (long long)(n - a.seg0) * D.n_vals + U.vb; };
+      // f -= value in the registers of a mask, values from v on.
+      auto add = [&](T (&f)[R][V], unsigned mask, int& v) {
+        if (flags & 128) {
+          const T* q = in_memory() + v;
 #pragma unroll
           for (int r = 0; r < R; ++r)
 #pragma unroll
             for (int k = 0; k < V; ++k)
-              if (p.reg() == r * V + k) {
-                if (p.kind() == 0)
-                  hx[r][k] += -v;
-                else
-                  hy[r][k] += -v;
-              }
+              if (mask >> (r * V + k) & 1) f[r][k] += -__ldg(q++);
+        } else {
+          const T* q = staged + v;
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+              if (mask >> (r * V + k) & 1) f[r][k] += -*q++;
+        }
+        v += __popc(mask);
+      };
+      if (flags & 1) {  // Mx / My
+        const RHdr& hd = D.hdr[(long long)tl.slot * S::NT + threadIdx.x];
+        unsigned mx = hd.m_hx, my = hd.m_hy;
+        int v = int(hd.v);
+#pragma unroll 1
+        for (int q = hd_first;; ++q) {
+          add(hx, mx, v);
+          add(hy, my, v);
+          if (!(flags & 256) || q >= at_jz()) break;
+          const RPt p = entry(q);
+          mx = unsigned(p.m);
+          my = p.w;
+          if (!(mx | my)) break;
         }
       }
       sts(sm + S::O_Y + row, hy[R - 1]);
@@ -960,22 +972,22 @@ __device__ __forceinline__ void body(const RDev<typename S::T>& D, const RTile& 
       if (flags & 31) {
         // Jz (fdtd2d.py:444), then the RVS ports' injections, then their V for
         // owned records (fdtd2d.py:446-451).
-        int inj = at_jz();
-        if ((flags & 258) == 258) {  // Jz, one a cell at most
+        if (flags & 2) {
           const RHdr& hd = D.hdr[(long long)tl.slot * S::NT + threadIdx.x];
-          const T* v = staged + hd.v_e;
-          const unsigned me = hd.m_e;
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int k = 0; k < V; ++k)
-              if (me >> (r * V + k) & 1) e[r][k] += -*v++;
-          inj = at_port();
+          unsigned me = hd.m_e;
+          int v = int(hd.v + (n01 & 0xffff));
+#pragma unroll 1
+          for (int q = at_jz();; ++q) {
+            add(e, me, v);
+            if (!(flags & 1024) || q >= at_port()) break;
+            me = unsigned(entry(q).m);
+            if (!me) break;
+          }
         }
-        if (flags & 6) {
-          for (int q = inj; q < at_probe(); ++q) {
+        if (flags & 4) {
+          for (int q = at_port(); q < at_probe(); ++q) {
             const RPt p = entry(q);
-            const T v = value(p.val());
+            const T v = p.val() < U.nvs ? staged[p.val()] : in_memory()[p.val()];
 #pragma unroll
             for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -1133,21 +1145,23 @@ __global__ void tm_headers(const RHdr* in, const int* at, int n, RHdr* out) {
   if (q < n) out[at[q]] = in[q];
 }
 
-// Injected values of steps [seg0, seg0 + cnt): one thread per injection and
-// FOLD steps (blockIdx.y). The products are formed like
-// the tile kernels' (src_term, mx_term, my_term and the port term).
+// Injected values of steps [seg0, seg0 + cnt): one thread per value and FOLD steps
+// (blockIdx.y). The products are formed like the tile kernels' (src_term, mx_term,
+// my_term and the port term), for every rectangle that an injection reaches, in the
+// order in which the rectangles read them.
 template <typename T>
 __global__ void __launch_bounds__(128) tm_values(const RDev<T>* dev, int seg0, int seg) {
   const RDev<T>& D = *dev;
   const Dev<T>& d = D.d;
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= D.n_inj) return;
+  if (id >= D.n_vals) return;
+  const int inj = D.vl[id];
   const int t0 = blockIdx.y * FOLD;
   const int cnt = min(FOLD, min(seg, d.n_steps - seg0) - t0);
-  T* const out = const_cast<T*>(D.pv) + (long long)t0 * D.n_inj + id;
+  T* const out = const_cast<T*>(D.pv) + (long long)t0 * D.n_vals + id;
   for (int t = 0; t < cnt; ++t) {
     const int n = seg0 + t0 + t;
-    int m = id;
+    int m = inj;
     T v;
     if (m < d.n_src) {
       v = src_term(d, m, n);
@@ -1159,7 +1173,7 @@ __global__ void __launch_bounds__(128) tm_values(const RDev<T>* dev, int seg0, i
       m -= d.n_my;
       v = d.cb_vs[m] * d.port_vs[(long long)n * d.n_ports + m];
     }
-    out[(long long)t * D.n_inj] = v;
+    out[(long long)t * D.n_vals] = v;
   }
 }
 
