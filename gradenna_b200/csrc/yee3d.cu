@@ -11,7 +11,7 @@
 // only E and the E kernel only H, so no CTA ever reads a value another CTA is
 // writing). A thread owns 16 bytes of cells along k (four float, two double) of
 // a row, a CTA 128 such vectors that follow one another over a plane's rows (no
-// lane is lost to nz), on two i-planes: the curl, update and padding work is
+// lane is lost to nz), on one to eight i-planes: the curl, update and padding work is
 // paid per vector load, the z slabs of all cells of a vector in one pass. All
 // operands of a plane, psi included, are loaded before the first use. CPML psi
 // lives in full padded volumes (zero outside the slabs) indexed like the
@@ -1113,12 +1113,17 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, c
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Planes per CTA for a step kernel: as few as let every CTA of the `cols`
-// column blocks be resident at once, two at most (more only where the planes
-// would be too many for a grid's second extent). Each plane is a trip to L2
-// that only other warps hide: at 160 x 160 x 64 f32 a step with 7 planes a CTA
-// (one wave) takes 53 us, with two (three waves) 50, with one 54; at 97 x 83 x
-// 61 four planes instead of two cost a quarter more.
+// Planes per CTA for a step kernel, 1 to 8 (more only where the planes would be too
+// many for a grid's second extent). A plane is a trip to L2 that only other warps
+// hide, so a wave of resident CTAs takes about as long as its planes, and a little
+// for the values carried into the first: the fewest waves x (planes + 0.4). ms for
+// 200 steps, two planes wherever one wave does not hold one each -> this rule (one
+// cell a thread, walking one wave):
+//   64 x 64 x 64 f64, CPML 6     4.75 -> 4.13 (4.38)
+//   97 x 83 x 61 f64, CPML 6     5.95 -> 5.33 (5.79)
+//   160 x 160 x 64 f64, CPML 6  16.6 -> 15.8 (16.5)
+//   100 x 100 x 100 f32, CPML 6  5.63 -> 5.39 (8.96)
+//   200 x 30 x 120 f32, no CPML  4.79 -> 4.10 (4.30)
 template <typename K>
 static int planes_per_cta(K kernel, int nx, int cols, int* ni) {
   int dev = 0, sms = 0, per_sm = 0;
@@ -1126,8 +1131,14 @@ static int planes_per_cta(K kernel, int nx, int cols, int* ni) {
   GDN_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   GDN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, 0));
   const long long slots = (long long)std::max(sms, 1) * std::max(per_sm, 1);
-  const long long per_col = std::max<long long>(1, slots / std::max(cols, 1));
-  *ni = int(std::min<long long>(2, std::max<long long>(1, div_up(nx, per_col))));
+  long long best = 0;
+  for (int q = 1; q <= 8; ++q) {
+    const long long cost = div_up(std::max(cols, 1) * div_up(nx, q), slots) * (10 * q + 4);
+    if (q == 1 || cost < best) {
+      best = cost;
+      *ni = q;
+    }
+  }
   *ni = int(std::max<long long>(*ni, div_up(nx, 65535)));
   return GDN_OK;
 }
