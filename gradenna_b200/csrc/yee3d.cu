@@ -442,12 +442,22 @@ __global__ void yee_pad_coef(Dev3<T> d, T* cap, T* cbp) {
   }
 }
 
+// CTAs an SM of the step kernels. Runs without CPML have kernels of their own: no
+// psi, masks or coefficients, so that six CTAs fit (80 registers, no spills) and
+// hide more of the loads' latency. ms for 200 steps, general kernels -> these (one
+// cell a thread): 160 x 160 x 64 f32 6.56 -> 4.72 (6.14), f64 12.9 -> 9.2 (11.1);
+// 30 x 200 x 120 f64 5.78 -> 4.47 (5.26); 97 x 83 x 61 f64 4.61 -> 3.86 (4.19).
+template <typename T>
+constexpr int step_ctas(bool pml) {
+  return pml ? (sizeof(T) == 4 ? 4 : 3) : 6;
+}
+
 // ---------------------------------------------------------------------------
 // H update: E^n -> H^{n+1/2} (fdtd3d.py:564-588). A CTA covers NT vectors of a
 // plane's rows and `ni` consecutive planes.
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, int ni) {
+template <typename T, bool PML>
+__global__ void __launch_bounds__(NT, step_ctas<T>(PML)) yee_h(Dev3<T> d, int ni) {
   constexpr int V = Vec<T>::V;
   constexpr unsigned ALL = (1u << V) - 1;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -462,10 +472,14 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, i
   T *hx = d.f[3], *hy = d.f[4], *hz = d.f[5];
   const T dt_mu = d.dt_mu, idx = d.inv_d[0], idy = d.inv_d[1], idz = d.inv_d[2];
   // This thread's y and z CPML samples (H-type) are fixed over the planes.
-  const Ax<T> ay = coef_at<T, false>(d, 1, th.live ? th.j : 0);
-  const Az<T> az = coef_z<T, false>(d, th.k0);
-  const bool yon = in_slab(d.npml, th.j, ny - 1);
-  const unsigned zon = slab_mask<V>(d.npml, th.k0, nz - 1);
+  Ax<T> ay{};
+  Az<T> az{};
+  if constexpr (PML) {
+    ay = coef_at<T, false>(d, 1, th.live ? th.j : 0);
+    az = coef_z<T, false>(d, th.k0);
+  }
+  const bool yon = PML && in_slab(d.npml, th.j, ny - 1);
+  const unsigned zon = PML ? slab_mask<V>(d.npml, th.k0, nz - 1) : 0u;
   const bool jin = th.j < ny - 1;
   const unsigned kin = range_mask<V>(th.k0, 0, nz - 1), kall = range_mask<V>(th.k0, 0, nz);
   // The tables are older than the chunk: only what follows needs the previous
@@ -482,7 +496,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, i
     const bool iin = i < nx - 1;
     const unsigned vx = jin ? kin : 0u, vy = iin ? kin : 0u, vz = iin && jin ? kall : 0u;
     // psi and the plane's x coefficients with the fields, before any use.
-    const bool xon = in_slab(d.npml, i, nx - 1);
+    const bool xon = PML && in_slab(d.npml, i, nx - 1);
     const unsigned o_xz = vx & zon, o_xy = yon ? vx : 0u, o_yx = xon ? vy : 0u, o_yz = vy & zon,
                    o_zy = yon ? vz : 0u, o_zx = xon ? vz : 0u;
     T* const psi = d.psi + c;
@@ -505,7 +519,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, i
       d4[x] = sub_(exj[x], ex0[x]);
       d5[x] = sub_(eyi[x], ey0[x]);
     }
-    const unsigned gen = near_slab(d.npml, i, i + 1, nx) ? ALL : th.gen;
+    const unsigned gen = !PML ? 0u : near_slab(d.npml, i, i + 1, nx) ? ALL : th.gen;
     if ((gen | (ALL ^ kin)) == 0 && iin && jin) {
       // No slab within reach and every cell live: the bare update.
 #pragma unroll
@@ -562,8 +576,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_h(Dev3<T> d, i
 // E update: H^{n+1/2} -> E^{n+1} (fdtd3d.py:596-633) + the sources near probes
 // and the port, the port, probes and V/I. Same CTA geometry as yee_h.
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_e(Dev3<T> d, int sub, int ni) {
+template <typename T, bool PML>
+__global__ void __launch_bounds__(NT, step_ctas<T>(PML)) yee_e(Dev3<T> d, int sub, int ni) {
   constexpr int V = Vec<T>::V;
   constexpr unsigned ALL = (1u << V) - 1;
   __shared__ T s_port[3];  // Ez^n, curl_z and the plain-updated Ez at the port edge
@@ -579,10 +593,14 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_e(Dev3<T> d, i
   const T* __restrict__ hz = d.f[5];
   const T idx = d.inv_d[0], idy = d.inv_d[1], idz = d.inv_d[2];
   // E-type samples of this thread's y and z (the PEC interior, node - 1).
-  const Ax<T> ay = coef_at<T, true>(d, 1, th.live ? th.j : 0);
-  const Az<T> az = coef_z<T, true>(d, th.k0);
-  const bool yon = in_slab(d.npml, th.j - 1, ny - 2);
-  const unsigned zon = slab_mask<V>(d.npml, th.k0 - 1, nz - 2);
+  Ax<T> ay{};
+  Az<T> az{};
+  if constexpr (PML) {
+    ay = coef_at<T, true>(d, 1, th.live ? th.j : 0);
+    az = coef_z<T, true>(d, th.k0);
+  }
+  const bool yon = PML && in_slab(d.npml, th.j - 1, ny - 2);
+  const unsigned zon = PML ? slab_mask<V>(d.npml, th.k0 - 1, nz - 2) : 0u;
   const bool jx = th.j >= 1 && th.j <= ny - 2;
   const unsigned kx = range_mask<V>(th.k0, 1, nz - 1), kin = range_mask<V>(th.k0, 0, nz - 1);
   dependent_launch_gate();  // the tables are older than the chunk
@@ -618,7 +636,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_e(Dev3<T> d, i
       const unsigned vx = i < nx - 1 && jx ? kx : 0u, vy = iin && th.j < ny - 1 ? kx : 0u,
                      vz = iin && jx ? kin : 0u;
       // psi and the plane's x coefficients with the fields, before any use.
-      const bool xon = in_slab(d.npml, i - 1, nx - 2);
+      const bool xon = PML && in_slab(d.npml, i - 1, nx - 2);
       const unsigned o_xy = yon ? vx : 0u, o_xz = vx & zon, o_yz = vy & zon, o_yx = xon ? vy : 0u,
                      o_zx = xon ? vz : 0u, o_zy = yon ? vz : 0u;
       T* const psi = d.psi + c;
@@ -643,7 +661,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3) yee_e(Dev3<T> d, i
       }
       Vec<T> old, curl;
       if (port_here) old = e2;
-      const unsigned gen = near_slab(d.npml, i, i + 1, nx) ? ALL : th.gen;
+      const unsigned gen = !PML ? 0u : near_slab(d.npml, i, i + 1, nx) ? ALL : th.gen;
       if ((gen | (ALL ^ kx)) == 0 && iin && jx) {
         // No slab within reach and every cell live: the bare update.
 #pragma unroll
@@ -1428,8 +1446,10 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
 
   const dim3 blk(NT);
   int ni_h = 0, ni_e = 0;
-  if ((st = planes_per_cta(yee_h<T>, nx, L.cols, &ni_h))) return st;
-  if ((st = planes_per_cta(yee_e<T>, nx, L.cols, &ni_e))) return st;
+  auto* const step_h = p->npml > 0 ? yee_h<T, true> : yee_h<T, false>;
+  auto* const step_e = p->npml > 0 ? yee_e<T, true> : yee_e<T, false>;
+  if ((st = planes_per_cta(step_h, nx, L.cols, &ni_h))) return st;
+  if ((st = planes_per_cta(step_e, nx, L.cols, &ni_e))) return st;
   const dim3 grd_h(unsigned(L.cols), unsigned(div_up(nx, ni_h)));
   const dim3 grd_e(unsigned(L.cols), unsigned(div_up(nx, ni_e)));
   const int eblocks = int(std::min<long long>(div_up((long long)nx * ny * nz, 256), 148 * 8));
@@ -1469,7 +1489,7 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
     const unsigned gb0 = unsigned(div_up(d.gcells[0], 256)), gb1 = unsigned(div_up(d.gcells[1], 256));
     for (int t = 0; t < cnt; ++t) {
       settle(pend_h, 1);
-      launch(yee_h<T>, grd_h, blk, s, d, ni_h);
+      launch(step_h, grd_h, blk, s, d, ni_h);
       k += 1;
       if (d.n_fp[1] > 0) {
         launch(yee_inject<T>, dim3(unsigned(div_up(d.n_fp[1], 256))), dim3(256), s, d, t, 1);
@@ -1480,7 +1500,7 @@ static int run3(const GdnYeeParams* p, const GdnYeePoints* pts, const GdnYeeBuff
         ++k;
       }
       settle(pend_e, 0);
-      launch(yee_e<T>, grd_e, blk, s, d, t, ni_e);
+      launch(step_e, grd_e, blk, s, d, t, ni_e);
       k += 1;
       if (d.n_fp[0] > 0) {
         launch(yee_inject<T>, dim3(unsigned(div_up(d.n_fp[0], 256))), dim3(256), s, d, t, 0);
