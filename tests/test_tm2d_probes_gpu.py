@@ -44,8 +44,12 @@ def test_blocks_of_probes(n, kind, dtype, monkeypatch):
             t.append(_native.tm_loop_stats(reset=True)[0])
         return min(t), r.probe_ez
 
-    mine, got = best()
-    monkeypatch.setenv("GDN_TM_KERNEL", "tile")
-    tile, want = best()
-    assert torch.equal(want, got)
-    assert mine <= 1.05 * tile  # the same kernels where a rectangle is crowded
+    for _ in range(3):  # another process on the host can disturb a try
+        mine, got = best()
+        with monkeypatch.context() as m:
+            m.setenv("GDN_TM_KERNEL", "tile")
+            tile, want = best()
+        assert torch.equal(want, got)
+        if mine <= 1.05 * tile:  # the same kernels where a rectangle is crowded
+            return
+    assert mine <= 1.05 * tile
