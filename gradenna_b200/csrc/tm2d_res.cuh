@@ -35,10 +35,10 @@
 // and ring stores.
 // Measured on B200 against the tile kernels alone, whole calls:
 //   70 x 53 f32, 300 steps, 2 frequencies                  2.8 ms -> 1.5 ms
-//   140 x 140 f32 gradient, 2 x 3500 steps                41.9 ms -> 19.7 ms
-//   280 x 280 f64 gradient, 2 x 7000 steps                  84 ms -> 53 ms
-//   517 x 384 f32, 2000 steps, 8 frequencies, whole grid  18.3 ms -> 9.6 ms
-//   1024 x 1024 f32 gradient, 2 x 8000 steps               143 ms -> 98 ms
+//   140 x 140 f32 gradient, 2 x 3500 steps                41.9 ms -> 20.1 ms
+//   280 x 280 f64 gradient, 2 x 7000 steps                  84 ms -> 54 ms
+//   517 x 384 f32, 2000 steps, 8 frequencies, whole grid  18.3 ms -> 9.7 ms
+//   1024 x 1024 f32 gradient, 2 x 8000 steps               143 ms -> 100 ms
 #pragma once
 
 namespace res {
